@@ -17,9 +17,12 @@
 // the same problem alone to rounding, and with the reference within the
 // solver tolerance.
 #pragma once
+#include <type_traits>
+
 #include "boundary.cuh"
 #include "common.cuh"
 #include "multigrid.cuh"
+#include "pattern.cuh"
 #include "poisson.cuh"
 #include "stencil.cuh"
 
@@ -54,6 +57,10 @@ struct BHier {
   int fused;        // levels 1..tail_level carry their fused restriction M
   int agg2;         // level 1 aggregates 2 x 2 fine cells: shape (ceil(nx/2), ceil(ny/2))
   int sp0, spn;     // this structure's problems: sprobs[sp0 .. sp0 + spn)
+  // the cycle above the tail as row patterns (pattern.cuh): dn[l] restricts onto level
+  // l, up[l] closes level l on the way up; ld, lu: parts a row is split into
+  Pat<T> dn[kBMaxLevels], up[kBMaxLevels];
+  int ld[kBMaxLevels], lu[kBMaxLevels];
 };
 
 // Device record of one problem.  T is the storage type of the (inner) CG and
@@ -71,6 +78,7 @@ struct BProb {
   int s_segs, s_items, s_chunks;         // warp strips of the solver kernels (b_strips)
   int vec, v_chunks;                     // vector strips (b_vstrips) in force; their blocks
   int p_chunks;                          // warp-strip chunks of the predictor (ghosted arrays)
+  int u_chunks;                          // row blocks of the level-0 up product (k_b_up0)
   int h_tr, h_tiles_j, h_tiles;          // staged tiles of the level-0 stencil transfers: rows, tiles
   int red_base;                          // first partial row of this problem
   const uint8_t* flags;
@@ -2027,6 +2035,327 @@ __global__ void __launch_bounds__(kBThreads, PCFD_BELL_MINB) k_b_ellg(const BPro
     case 8: b_ellg_rows<8, OP, GS>(P0, fw, flags0, G, E, wd, d, rb); break;
     case 16: b_ellg_rows<16, OP, GS>(P0, fw, flags0, G, E, wd, d, rb); break;
     default: b_ellg_rows<32, OP, GS>(P0, fw, flags0, G, E, wd, d, rb); break;
+  }
+}
+
+// ---- pattern products: the V-cycle above the tails ---------------------------------
+// One sweep per level, every structure tailed: a depth's down product b_d = M_d b_{d-1}
+// and up product x_d = Q_d x_{d+1} + G_d b_d (pattern.cuh) are one launch each over every
+// structure.  A block applies 256 / L rows of a structure's operator to a group of its
+// problems: a row's entries are read from the pattern table once for the group, its
+// gathers run along y over adjacent rows, and L > 1 splits the entries of the wide,
+// short levels over L parts of the block (each warp still covers 32 adjacent rows).
+// What bounds these launches is latency (dependent loads at the start of a block, gathers
+// at 40 % of the warp slots) and, at level 0, the instructions per gather; the grouped ELL
+// phases they replace read 8 bytes per entry and row from L2 with the row's entries spread
+// over a warp.  Per launch on 256 cavities in one engine (us): down onto level 1 60 -> 35,
+// onto 2 30 -> 22; level 1 up 76 (two launches) -> 37, level 2 up 58 -> 27; level 0 with
+// its last sweep 109 (two launches) -> 68.
+constexpr int kPatPart = 12;    // entries a part of a row takes at least
+constexpr int kPatMaxL = 8;     // parts of a row at most
+inline int pat_parts(int K) {
+  int L = 1;
+  while (L < kPatMaxL && K / (2 * L) >= kPatPart) L *= 2;
+  return L;
+}
+
+// One block of an operator (its second source s2 when TWO): sums of rows
+// [rb * 256 / L, ...) for GS members, handed to put(g, row, sum) with every member's
+// rows spread over the parts.
+template <bool TWO, int GS, class T, class Put>
+__device__ __forceinline__ void b_pat_rows(const Pat<T>& E, const T* const (&s1)[GS], const T (&sh1)[GS],
+                                           const T* const (&s2)[GS], int L, int rb, Put put) {
+  const int rpb = kBThreads / L;
+  const int part = (int)threadIdx.x / rpb, rl = (int)threadIdx.x - part * rpb;
+  const int row = rb * rpb + rl;
+  const int K = E.K + (TWO ? E.K2 : 0);
+  const int per = (K + L - 1) / L, k0 = part * per, k1 = min(K, k0 + per);
+  T acc[GS];
+#pragma unroll
+  for (int g = 0; g < GS; ++g) acc[g] = (T)0;
+  if (row < E.n) {
+    const PatEntry<T>* tb = E.tab + (long)E.pid[row] * K;
+    if (k0 < E.K)
+      pat_entries<GS, 0, !TWO>(tb + k0, min(k1, E.K) - k0, pat_base(E, row), s1, sh1, acc);
+    if (TWO && k1 > E.K) {
+      const int q = max(k0, E.K);
+      pat_entries<GS, 0, false>(tb + q, k1 - q, row, s2, sh1, acc);
+    }
+  }
+  if (L == 1) {
+    if (row < E.n) {
+#pragma unroll
+      for (int g = 0; g < GS; ++g) put(g, row, acc[g]);
+    }
+    return;
+  }
+  __shared__ T red[GS][kBThreads];
+#pragma unroll
+  for (int g = 0; g < GS; ++g) red[g][threadIdx.x] = acc[g];
+  __syncthreads();
+  if (row >= E.n) return;
+  for (int g = part; g < GS; g += L) {   // a part adds its members' sums, in part order
+    T t = red[g][rl];
+    for (int q = 1; q < L; ++q) t += red[g][q * rpb + rl];
+    put(g, row, t);
+  }
+}
+
+// The solving members of a block's group, packed to the front; the slots behind them
+// repeat the first member's sources and have no output.
+template <class T, int GS>
+struct BPatGroup {
+  const T* a[GS];    // gathered by the first operator
+  const T* b[GS];    // gathered by the second
+  T* out[GS];
+  T mr[GS];          // mean removed from a gathered level-0 residual
+  int pi[GS];
+  int n;
+};
+// Filled by warp 0 (every lane calls it): lane k < GS offers problem pi (-1: none).
+template <class T, int GS>
+__device__ __forceinline__ void b_pat_pack(BPatGroup<T, GS>& G, int pi, const T* a, const T* b, T* o, T mr) {
+  const int lane = (int)threadIdx.x;
+  const unsigned on = __ballot_sync(0xffffffffu, pi >= 0);
+  const int n = __popc(on);
+  if (pi >= 0) {
+    const int at = __popc(on & ((1u << lane) - 1u));
+    G.a[at] = a;
+    G.b[at] = b;
+    G.out[at] = o;
+    G.mr[at] = mr;
+    G.pi[at] = pi;
+  }
+  if (lane == 0) G.n = n;
+  __syncwarp();
+  if (n && lane >= n && lane < GS) {
+    G.a[lane] = G.a[0];
+    G.b[lane] = G.b[0];
+    G.out[lane] = nullptr;
+    G.mr[lane] = (T)0;
+    G.pi[lane] = -1;
+  }
+}
+// f(integral_constant<GS>) with the smallest of 1, 2, 4, 8 slots that holds n members.
+template <int GSMAX, class F>
+__device__ __forceinline__ void b_pat_width(int n, F f) {
+  if constexpr (GSMAX >= 8) {
+    if (n > 4) return f(std::integral_constant<int, 8>{});
+  }
+  if (n > 2) return f(std::integral_constant<int, 4>{});
+  if (n > 1) return f(std::integral_constant<int, 2>{});
+  f(std::integral_constant<int, 1>{});
+}
+template <class T, int GM, int GS>
+__device__ __forceinline__ void b_pat_copy(const BPatGroup<T, GM>& G, const T* (&a)[GS], const T* (&b)[GS],
+                                           T (&mr)[GS]) {
+#pragma unroll
+  for (int g = 0; g < GS; ++g) {
+    a[g] = G.a[g];
+    b[g] = G.b[g];
+    mr[g] = G.mr[g];
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kBThreads, sizeof(T) == 4 ? 4 : 3) k_b_down(const BProb<T>* __restrict__ probs,
+                                                         const BHier<T>* __restrict__ hiers,
+                                                         const int2* __restrict__ map,
+                                                         const int* __restrict__ sprobs, int d, BShared sh) {
+  pdl_begin();   // programmatic dependent launch: the predecessor's results first
+  constexpr int GM = kBGroup;
+  const int2 e = map[blockIdx.x];   // (structure, row block x 1024 + group)
+  const BHier<T>& H = hiers[e.x];
+  __shared__ BPatGroup<T, GM> G;
+  const Pat<T> E = H.dn[d];
+  const int L = H.ld[d];
+  if (threadIdx.x < 32) {
+    const int k = (e.y & 1023) * GM + (int)threadIdx.x;
+    int pi = (int)threadIdx.x < GM && k < H.spn ? sprobs[H.sp0 + k] : -1;
+    if (pi >= 0 && !b_solving(sh, pi)) pi = -1;
+    const T* a = nullptr;
+    T* o = nullptr;
+    T mr = (T)0;
+    if (pi >= 0) {
+      const BProb<T>& P = probs[pi];
+      a = d == 1 ? P.r : P.lb[d - 1];
+      o = P.lb[d];
+      if (d == 1 && P.singular) mr = (T)P.S[S_MEAN_R];
+    }
+    b_pat_pack<T, GM>(G, pi, a, a, o, mr);
+  }
+  __syncthreads();
+  if (!G.n) return;
+  b_pat_width<GM>(G.n, [&](auto w) {
+    constexpr int GS = decltype(w)::value;
+    const T *a[GS], *b[GS];
+    T mr[GS];
+    b_pat_copy(G, a, b, mr);
+    b_pat_rows<false, GS, T>(E, a, mr, b, L, e.y >> 10, [&](int g, int row, T v) {
+      if (G.out[g]) G.out[g][row] = v;
+    });
+  });
+}
+
+// x_d = Q_d x_{d+1} + G_d b_d at a coarse depth d >= 1.
+template <class T>
+__global__ void __launch_bounds__(kBThreads, sizeof(T) == 4 ? 4 : 3) k_b_up(const BProb<T>* __restrict__ probs,
+                                                       const BHier<T>* __restrict__ hiers,
+                                                       const int2* __restrict__ map,
+                                                       const int* __restrict__ sprobs, int d, BShared sh) {
+  pdl_begin();   // programmatic dependent launch: the predecessor's results first
+  constexpr int GM = kBGroup;
+  const int2 e = map[blockIdx.x];   // (structure, row block x 1024 + group)
+  const BHier<T>& H = hiers[e.x];
+  __shared__ BPatGroup<T, GM> G;
+  const Pat<T> E = H.up[d];
+  const int L = H.lu[d];
+  if (threadIdx.x < 32) {
+    const int k = (e.y & 1023) * GM + (int)threadIdx.x;
+    int pi = (int)threadIdx.x < GM && k < H.spn ? sprobs[H.sp0 + k] : -1;
+    if (pi >= 0 && !b_solving(sh, pi)) pi = -1;
+    const T *a = nullptr, *b = nullptr;
+    T* o = nullptr;
+    if (pi >= 0) {
+      const BProb<T>& P = probs[pi];
+      a = P.lxa[d + 1];
+      b = P.lb[d];
+      o = P.lxa[d];
+    }
+    b_pat_pack<T, GM>(G, pi, a, b, o, (T)0);
+  }
+  __syncthreads();
+  if (!G.n) return;
+  b_pat_width<GM>(G.n, [&](auto w) {
+    constexpr int GS = decltype(w)::value;
+    const T *a[GS], *b[GS];
+    T none[GS];
+    b_pat_copy(G, a, b, none);
+#pragma unroll
+    for (int g = 0; g < GS; ++g) none[g] = (T)0;
+    b_pat_rows<true, GS, T>(E, a, none, b, L, e.y >> 10, [&](int g, int row, T v) {
+      if (G.out[g]) G.out[g][row] = v;
+    });
+  });
+}
+
+// Level 0: z = Q_0 x_1 + G_0 b_0 (b_0 the projected CG residual), with sum z and r.z per
+// problem.  kUpRounds blocks of 256 rows for kUpGroup problems per block, so that the
+// block's sums (two per member) are closed once for 2048 rows of each problem.
+constexpr int kUpGroup = 4;
+constexpr int kUpRounds = 8;
+template <class T>
+__global__ void __launch_bounds__(kBThreads, 3)
+    k_b_up0(const BProb<T>* __restrict__ probs, const BHier<T>* __restrict__ hiers, const int2* __restrict__ map,
+            const int* __restrict__ sprobs, BShared sh) {
+  pdl_begin();   // programmatic dependent launch: the predecessor's results first
+  constexpr int GM = kUpGroup;
+  const int2 e = map[blockIdx.x];   // (structure, row block x 4096 + group)
+  const BHier<T>& H = hiers[e.x];
+  __shared__ BPatGroup<T, GM> G;
+  __shared__ unsigned closing;
+  const Pat<T> E = H.up[0];
+  const bool usual = E.K == 6 && E.K2 == 5;   // 2 x 2 aggregates of the five-point operator
+  const int KT = E.K + E.K2;
+  const int rb = e.y >> 12;
+  const uint8_t* __restrict__ flags = probs[sprobs[H.sp0]].flags;   // the structure's
+  if (threadIdx.x < 32) {
+    const int k = (e.y & 4095) * GM + (int)threadIdx.x;
+    int pi = (int)threadIdx.x < GM && k < H.spn ? sprobs[H.sp0 + k] : -1;
+    if (pi >= 0 && !b_solving(sh, pi)) pi = -1;
+    const T *a = nullptr, *b = nullptr;
+    T* o = nullptr;
+    T mr = (T)0;
+    if (pi >= 0) {
+      const BProb<T>& P = probs[pi];
+      a = P.lxa[1];
+      b = P.r;
+      o = P.z;
+      if (P.singular) mr = (T)P.S[S_MEAN_R];
+    }
+    b_pat_pack<T, GM>(G, pi, a, b, o, mr);
+  }
+  __syncthreads();
+  if (!G.n) return;
+  double sum[2 * GM];
+#pragma unroll
+  for (int g = 0; g < 2 * GM; ++g) sum[g] = 0.0;
+  const int row1 = min(E.n, (rb + 1) * kUpRounds * kBThreads);
+  b_pat_width<GM>(G.n, [&](auto w) {
+    constexpr int GS = decltype(w)::value;
+    const T *a[GS], *b[GS];
+    T mr[GS];
+    b_pat_copy(G, a, b, mr);
+    int row = rb * kUpRounds * kBThreads + (int)threadIdx.x;
+    int pid = row < row1 ? E.pid[row] : 0;
+    uint8_t fl = row < row1 ? flags[row] : 0;
+    for (; row < row1; row += kBThreads) {
+      const PatEntry<T>* tb = E.tab + (long)pid * KT;
+      const bool solv = (fl & F_SOLV) != 0;
+      const int nx = row + kBThreads;   // the next row's pattern, ahead of its use
+      if (nx < row1) {
+        pid = E.pid[nx];
+        fl = flags[nx];
+      }
+      T acc[GS], own[GS];
+#pragma unroll
+      for (int g = 0; g < GS; ++g) {
+        acc[g] = (T)0;
+        own[g] = b[g][row];
+      }
+      if (usual) {
+        pat_entries<GS, 6, false>(tb, 6, pat_base(E, row), a, mr, acc);
+        pat_entries<GS, 5, true>(tb + 6, 5, row, b, mr, acc);
+      } else {
+        pat_entries<GS, 0, false>(tb, E.K, pat_base(E, row), a, mr, acc);
+        pat_entries<GS, 0, true>(tb + E.K, E.K2, row, b, mr, acc);
+      }
+#pragma unroll
+      for (int g = 0; g < GS; ++g) {
+        if (T* o = G.out[g]) o[row] = acc[g];
+        if (solv) {
+          sum[2 * g] += (double)acc[g];
+          sum[2 * g + 1] += (double)own[g] * (double)acc[g];
+        }
+      }
+    }
+  });
+  block_reduce<2 * GM>(sum);
+  // lane g of warp 0 stores member g's partials and takes its ticket
+  if (threadIdx.x < 32) {
+    bool last = false;
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int g = 0; g < GM; ++g)
+      if ((int)threadIdx.x == g) {
+        s0 = sum[2 * g];
+        s1 = sum[2 * g + 1];
+      }
+    if ((int)threadIdx.x < G.n) {
+      const BProb<T>& P = probs[G.pi[threadIdx.x]];
+      double* part = sh.partials + (long)P.red_base * 8 + (long)rb * 2;
+      part[0] = s0;
+      part[1] = s1;
+      __threadfence();
+      last = atomicAdd(P.counter, 1u) == (unsigned)P.u_chunks - 1;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, last);
+    if (threadIdx.x == 0) closing = m;
+  }
+  __syncthreads();
+  const unsigned todo = closing;   // members whose last block this is
+  if (!todo) return;
+  __threadfence();
+  for (int g = 0; g < GM; ++g) {
+    if (!((todo >> g) & 1u)) continue;
+    const BProb<T>& P = probs[G.pi[g]];
+    double t[2];
+    sum_partials<2>(sh.partials + (long)P.red_base * 8, P.u_chunks, (int)threadIdx.x, kBThreads, t);
+    block_reduce<2>(t);
+    if (threadIdx.x == 0) {
+      b_last_close(P, t);
+      *P.counter = 0u;
+    }
   }
 }
 

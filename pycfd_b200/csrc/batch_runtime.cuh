@@ -25,6 +25,8 @@ struct pycfd_batch {
   int fused = 0;                           // down sweep by fused restrictions (every structure has them)
   int fused_from = 1;                      // first level restricted by the fused product (1 or 2)
   int ell_group = kBGroup;                 // problems per block of the coarse-level launches (1 or kBGroup)
+  int pats = 0;                            // the cycle above the tails as pattern products
+  BMapHost map0;                           // level-0 up product: (structure, row block x 4096 + group of kUpGroup)
   int stencil_req = 0;                     // level-0 transfers as stencils, as asked
   int stencil = 0;                         // ... and in force (fused down sweep from the fine level)
   int scalar_strips = 0;                   // FP32 solver kernels on scalar strips even where rows allow vectors
@@ -74,10 +76,18 @@ int upload_map(pycfd_batch* B, BMapHost* m, const std::vector<int2>& h) {
   return upload(B->mem, &m->e, h.data(), h.size());
 }
 
+// The level whose cycle one dense operator closes under the pattern products: the dense
+// tail's, or the coarsest with its pseudo-inverse.
+inline int b_closed_at(const pycfd_solver_desc* d) {
+  return d->tail_level > 0 && d->tail_level < d->n_levels - 1 && d->tail_operator ? d->tail_level : d->n_levels - 1;
+}
+
 // Upload one structure's hierarchy (from the descriptor of its first problem)
 // in storage type T.
+// cyc: the pattern products of its levels (B->pats), which take the place of the ELL blocks.
 template <class T>
-int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, BHier<T>* H, std::vector<Level>* keep) {
+int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, const PatCycle<T>* cyc, BHier<T>* H,
+                std::vector<Level>* keep) {
   const int Lv = d->n_levels;
   keep->resize(Lv);
   H->nlev = Lv;
@@ -89,6 +99,7 @@ int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, BHier<T>* H, std::ve
     const pycfd_mg_level& up = d->levels[l - 1];
     Level& L = (*keep)[l];
     L.n = in.n;
+    if (cyc) continue;
     const bool coarsest = l == Lv - 1;
     DevEll<T> A, P, R;
     T* wd = nullptr;
@@ -121,18 +132,26 @@ int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, BHier<T>* H, std::ve
     bl.wd = wd;
     bl.n = in.n;
   }
-  if (B->coarse == 0 && d->tail_level > 0 && d->tail_level < Lv - 1 && d->tail_operator) {
-    const int nt = d->levels[d->tail_level].n;
+  const int t = b_closed_at(d);
+  if (cyc || (B->coarse == 0 && t < Lv - 1)) {
+    const int nt = d->levels[t].n;
+    const double* op = t < Lv - 1 ? d->tail_operator : d->coarsest_inverse;
     std::vector<T> m((size_t)nt * nt);
-    for (size_t e = 0; e < m.size(); ++e) m[e] = (T)d->tail_operator[e];
+    for (size_t e = 0; e < m.size(); ++e) m[e] = (T)op[e];
     T* md = nullptr;
     TRY(upload(B->mem, &md, m.data(), m.size()));
     H->tail = md;
-    H->tail_level = d->tail_level;
+    H->tail_level = t;
     H->tail_n = nt;
     H->fused = 1;
-    for (int l = 1; l <= d->tail_level; ++l)
+    for (int l = 1; l <= t; ++l)
       if (!d->levels[l].m_indptr) H->fused = 0;
+    for (int l = 0; cyc && l < t; ++l) {
+      TRY(pat_upload(B->mem, cyc->dn[l + 1], &H->dn[l + 1]));
+      TRY(pat_upload(B->mem, cyc->up[l], &H->up[l]));
+      H->ld[l + 1] = pat_parts(H->dn[l + 1].K);
+      H->lu[l] = pat_parts(H->up[l].K + H->up[l].K2);
+    }
   }
   const int nc = d->levels[Lv - 1].n;
   std::vector<T> c((size_t)nc * nc);
@@ -167,6 +186,22 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   }
   std::vector<BHier<T>> hh(leaders.size());
   std::vector<std::vector<Level>> keep(leaders.size());
+  // pattern products: one sweep per level and no option asking for another form of the
+  // cycle (the rule reads nothing of the other problems, so that a problem takes the
+  // same route in every split of a batch)
+  std::vector<PatCycle<T>> cyc(leaders.size());
+  B->pats = (B->coarse == 0 && B->sweeps == 1 && B->ell_group == kBGroup && B->fused_from == 1 && !B->stencil_req);
+  {
+    std::vector<std::function<bool()>> tasks;
+    for (size_t h = 0; B->pats && h < leaders.size(); ++h) {
+      const pycfd_solver_desc& d = descs[leaders[h]];
+      if (d.n_levels < 2 || d.n_levels > kBMaxLevels || !d.levels || !d.coarsest_inverse ||
+          d.levels[0].n != d.nx * d.ny ||
+          !pat_tasks<T>(d.levels, b_closed_at(&d), true, B->solvers[leaders[h]]->hflags.data(), &cyc[h], &tasks))
+        B->pats = 0;
+    }
+    if (B->pats && !run_tasks(tasks)) B->pats = 0;
+  }
   for (size_t h = 0; h < leaders.size(); ++h) {
     const pycfd_solver_desc& d = descs[leaders[h]];
     if (d.n_levels < 2 || !d.levels || !d.coarsest_inverse)
@@ -175,7 +210,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     if (d.n_levels > kBMaxLevels) return fail(PCFD_E_ARG, "at most %d multigrid levels", kBMaxLevels);
     if (d.levels[0].n != d.nx * d.ny) return fail(PCFD_E_ARG, "level 0 must have nx*ny unknowns");
     hh[h] = BHier<T>{};
-    TRY(upload_hier<T>(B, &d, &hh[h], &keep[h]));
+    TRY(upload_hier<T>(B, &d, B->pats ? &cyc[h] : nullptr, &hh[h], &keep[h]));
   }
   if (B->smem_dense > 48 * 1024)
     return fail(PCFD_E_UNSUPPORTED, "coarsest level too large for the one-block dense solve");
@@ -227,8 +262,9 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
       P.h_tiles_j = (s->g.ny + kBHaloTC - 1) / kBHaloTC;
       P.h_tiles = ((s->g.nx + tr - 1) / tr) * P.h_tiles_j;
     }
+    P.u_chunks = (s->g.nx * s->g.ny + kUpRounds * kBThreads - 1) / (kUpRounds * kBThreads);
     P.red_base = red_rows;
-    red_rows += std::max(std::max(P.chunks, std::max(P.s_chunks, P.v_chunks)), P.h_tiles);
+    red_rows += std::max({P.chunks, P.s_chunks, P.v_chunks, P.h_tiles, P.u_chunks});
     P.flags = s->flags;
     P.solid = s->solid;
     P.bc_kind = s->bc_kind_dev;
@@ -339,7 +375,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   B->mapR.assign(B->depth, BMapHost{});
   B->mapP.assign(B->depth, BMapHost{});
   B->mapC.assign(B->depth, BMapHost{});
-  std::vector<int2> mt;
+  std::vector<int2> mt, m0;
   for (int d = 0; d < B->depth; ++d) {
     std::vector<int2> ma, mr, mp, mc;
     for (size_t h = 0; h < leaders.size(); ++h) {
@@ -352,6 +388,23 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
         const int cts = (H.spn + kTailBN - 1) / kTailBN;
         for (int rt = 0; rt < rts; ++rt)
           for (int c = 0; c < cts; ++c) mt.push_back(make_int2((int)h, rt * 64 + c));
+      }
+      if (B->pats) {
+        if (d > H.tail_level) continue;
+        const int nrow = d == 0 ? pr[leaders[h]].g.nx * pr[leaders[h]].g.ny : keep[h][d].n;
+        if (d == 0) {
+          const int g4 = (H.spn + kUpGroup - 1) / kUpGroup;
+          for (int rb = 0; rb * kUpRounds * kBThreads < nrow; ++rb)
+            for (int g = 0; g < g4; ++g) m0.push_back(make_int2((int)h, rb * 4096 + g));
+          continue;
+        }
+        auto rows = [&](std::vector<int2>& m, int L) {
+          for (int rb = 0; rb * (kBThreads / L) < nrow; ++rb)
+            for (int g = 0; g < grps; ++g) m.push_back(make_int2((int)h, rb * 1024 + g));
+        };
+        rows(mr, H.ld[d]);
+        if (d < H.tail_level) rows(ma, H.lu[d]);
+        continue;
       }
       const int lead = leaders[h];
       const int c = B->nlev[lead] - 1;
@@ -392,6 +445,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     TRY(upload_map(B, &B->mapC[d], mc));
   }
   TRY(upload_map(B, &B->mapT, mt));
+  TRY(upload_map(B, &B->map0, m0));
   {
     std::vector<int> ord(n);
     for (int i = 0; i < n; ++i) ord[i] = i;
@@ -512,6 +566,25 @@ template <class T>
 int b_vcycle(pycfd_batch* B, cudaStream_t st) {
   const int sw = B->sweeps;
   const int D = B->coarse > 0 ? std::min(B->coarse, B->depth) : B->depth;   // depths run per level
+  if (B->pats) {   // down products, tails, up products: one launch per depth and direction
+    b_prof(B, 4, st);
+    for (int d = 1; d < D; ++d)
+      if (B->mapR[d].n)
+        BLAUNCH(k_b_down<T>, B->mapR[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapR[d].e, B->sprobs,
+                d, B->sh);
+    b_prof(B, 4, st);
+    TRY(b_tails<T>(B, st));
+    b_prof(B, 4, st);
+    for (int d = D - 1; d >= 1; --d)
+      if (B->mapA[d].n)
+        BLAUNCH(k_b_up<T>, B->mapA[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapA[d].e, B->sprobs, d,
+                B->sh);
+    b_prof(B, 4, st);
+    b_prof(B, 2, st);
+    BLAUNCH(k_b_up0<T>, B->map0.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->map0.e, B->sprobs, B->sh);
+    b_prof(B, 2, st);
+    return 0;
+  }
   if (B->fused) {
     // ---- down: b_d = M_d b_{d-1} at every depth from fused_from above each problem's
     // tail (below it the fine sweep and R), then the tails
@@ -860,7 +933,7 @@ int pycfd_batch_create(const pycfd_solver_desc* descs, const int* structure, con
     d.precision = opts->precision;
     d.tol = opts->tol;
     d.maxiter = opts->maxiter;
-    int rc = pycfd_solver_create(&d, &B->solvers[i]);
+    int rc = solver_create(&d, true, &B->solvers[i]);
     if (rc) return bail(rc);
   }
   int rc = opts->precision == PCFD_MIXED ? batch_build<float>(B, descs, structure, dt_ctl, max_steps, u, v, p)

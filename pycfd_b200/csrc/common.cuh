@@ -109,13 +109,17 @@ constexpr int kRedThreads = 256;
 
 // Programmatic dependent launch (sm_90+): a kernel launched with the
 // programmatic-serialization attribute may be scheduled while its predecessor
-// is still running.  Every kernel therefore first waits for the predecessor's
-// completion and memory (a no-op without the attribute), then allows its own
-// successor to be scheduled, so the launch latency between dependent kernels
-// overlaps execution.
+// is still running.  Every kernel therefore first allows its own successor to be
+// scheduled (which happens once all its blocks have started, so the successor takes
+// only what they leave free), then waits for the predecessor's completion and memory
+// (a no-op without the attribute): launch latency overlaps execution, and what a kernel
+// does between the two -- reading tables that no kernel writes -- overlaps its
+// predecessor.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait();
+  pdl_trigger();
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -13,6 +13,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "pattern.cuh"
 
 namespace pcfd {
 
@@ -302,6 +303,128 @@ __global__ void k_ell_prolong0_wb(Ell<T> P, B bf, const uint8_t* __restrict__ fl
   ell_pass<L>(P, [&](int c) { return (double)xc[c]; }, [&](int row, double s) {
     const int i = row / g.ny, j = row - i * g.ny;
     xf[row] = (T)((double)(T)(fine_wdinv(flags[row], i, j, g, w) * bf(row)) + s);
+  });
+}
+
+// ---- pattern products of one problem -------------------------------------------
+// Down and up products of the cycle above the dense tail (pattern.cuh), 256 / L rows per
+// block, a row's entries split over L parts of the block whose sums are added in part
+// order.  A single problem's levels are short, so the launch is bound by its chain of
+// dependent loads: the pattern and its first entries (tables no kernel writes) are read
+// before the wait for the predecessor, and one round of gathers is left behind it.
+constexpr int kPatChunk = 8;        // entries gathered together
+constexpr int kPatMaxParts = 32;
+// Parts per row: about three entries each, within the resident threads of the GPU.
+inline int pat_parts1(int n, int K, long threads) {
+  int L = 1;
+  while (L < kPatMaxParts && K >= 6 * L && (long)n * L * 2 <= threads) L *= 2;
+  return L;
+}
+
+// Sum of row `row` over entries [k0, k1): E's first source from its base, the second
+// from the row; `begin` runs between the first table reads and the first gather.
+template <class T, class Begin, class X1, class X2>
+__device__ __forceinline__ double pat_sum(const Pat<T>& E, int row, int k0, int k1, Begin begin, X1 x1, X2 x2) {
+  const bool ok = row < E.n && k0 < k1;
+  const int K = E.K + E.K2;
+  const int base = ok ? pat_base(E, row) : 0;
+  const PatEntry<T>* tb = E.tab + (ok ? (long)E.pid[row] * K : 0);
+  int at[kPatChunk];
+  T val[kPatChunk];
+  auto load = [&](int k) {
+#pragma unroll
+    for (int u = 0; u < kPatChunk; ++u) {
+      at[u] = 0;
+      val[u] = (T)0;
+      if (k + u < k1) {
+        pat_load(tb + k + u, &at[u], &val[u]);
+        at[u] += k + u < E.K ? base : row;
+      }
+    }
+  };
+  if (ok) load(k0);
+  begin();
+  double acc = 0.0;
+  if (!ok) return acc;
+  for (int k = k0;;) {
+    double x[kPatChunk];
+#pragma unroll
+    for (int u = 0; u < kPatChunk; ++u) x[u] = k + u < k1 ? (k + u < E.K ? x1(at[u]) : x2(at[u])) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kPatChunk; ++u) acc += (double)val[u] * x[u];
+    k += kPatChunk;
+    if (k >= k1) return acc;
+    load(k);
+  }
+}
+
+// y = E x1 (+ second source x2): FROM_R: the first source of a down product is the CG
+// residual less its fluid mean.
+template <class T, bool FROM_R>
+__global__ void __launch_bounds__(256) k_pat(Pat<T> E, int L, const T* __restrict__ s1, const T* __restrict__ s2,
+                                             const double* __restrict__ S, int singular, T* __restrict__ y) {
+  const int rpb = 256 / L;
+  const int part = (int)threadIdx.x / rpb, rl = (int)threadIdx.x - part * rpb;
+  const int row = (int)blockIdx.x * rpb + rl;
+  const int K = E.K + E.K2, per = (K + L - 1) / L, k0 = part * per, k1 = min(K, k0 + per);
+  double mean = 0.0;
+  const double acc = pat_sum(
+      E, row, k0, k1,
+      [&]() {
+        pdl_begin();
+        if (FROM_R && singular) mean = S[S_MEAN_R];
+      },
+      [&](int c) { return FROM_R ? (double)s1[c] - mean : (double)s1[c]; }, [&](int c) { return (double)s2[c]; });
+  if (L == 1) {
+    if (row < E.n) y[row] = (T)acc;
+    return;
+  }
+  __shared__ double red[256];
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  if (part == 0 && row < E.n) {
+    double t = acc;
+    for (int q = 1; q < L; ++q) t += red[q * rpb + rl];
+    y[row] = (T)t;
+  }
+}
+
+// Level 0: z = Q_0 x_1 + G_0 b_0 (b_0 the projected CG residual) with sum z and r.z for
+// the projected z and rho, one row per thread.
+template <class T>
+__global__ void __launch_bounds__(256) k_pat_up0(Pat<T> E, const T* __restrict__ x1, const T* __restrict__ r,
+                                                 const uint8_t* __restrict__ flags, Geo g, int singular,
+                                                 double* __restrict__ S, T* __restrict__ z, RedBuf rb) {
+  const int K = E.K + E.K2;
+  double acc[2] = {0, 0};
+  double mean = 0.0;
+  bool waited = false;
+  for (int row0 = (int)blockIdx.x * 256; row0 < E.n; row0 += (int)gridDim.x * 256) {
+    const int row = row0 + (int)threadIdx.x;
+    const uint8_t f = row < E.n ? flags[row] : 0;
+    const double v = pat_sum(
+        E, row, 0, K,
+        [&]() {
+          if (waited) return;
+          pdl_begin();
+          waited = true;
+          if (singular) mean = S[S_MEAN_R];
+        },
+        [&](int c) { return (double)x1[c]; }, [&](int c) { return (double)r[c] - mean; });
+    if (row < E.n) {
+      const double zn = (double)(T)v;
+      z[row] = (T)zn;
+      if (f & F_SOLV) {
+        acc[0] += zn;
+        acc[1] += (double)r[row] * zn;
+      }
+    }
+  }
+  grid_reduce<2>(acc, rb, [&](double* t) {
+    const double m = (singular && g.n_fluid) ? t[0] / g.n_fluid : 0.0;
+    S[S_MEAN_Z] = m;
+    S[S_RHO_PREV] = S[S_RHO];
+    S[S_RHO] = t[1] - m * S[S_SUM_R];
   });
 }
 

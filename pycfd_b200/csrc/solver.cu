@@ -7,8 +7,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
+#include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/pycfd_b200.h"
@@ -16,6 +19,7 @@
 #include "cluster.cuh"
 #include "common.cuh"
 #include "multigrid.cuh"
+#include "pattern.cuh"
 #include "persistent.cuh"
 #include "masks.cuh"
 #include "adjoint.cuh"
@@ -118,6 +122,7 @@ struct pycfd_solver {
   int singular = 1;
   std::vector<void*> allocs;
 
+  std::vector<uint8_t> hflags;  // host copy of the cell flags
   uint8_t* flags = nullptr;
   uint8_t* solid = nullptr;
   int* mask_u = nullptr;
@@ -148,6 +153,10 @@ struct pycfd_solver {
   int nc = 0;
   int tail_level = 0;           // level whose cycle is one dense operator (0: none)
   int fused = 0;                // down sweep by fused restrictions onto levels 1..tail_level
+  // the cycle above the tail as pattern products (empty: the ELL operators)
+  std::vector<Pat<double>> pdn, pup;
+  std::vector<Pat<float>> pdnf, pupf;
+  long pat_threads = 0;         // resident threads a pattern product spreads its rows over
   long ell_budget = 0;          // resident threads a per-phase ELL pass may use (< 0: storage lanes)
   int ell_blocks = kWaveBlocks; // grid cap of the per-phase ELL kernels
   double* tail = nullptr;
@@ -275,6 +284,10 @@ void csr_transpose(int nrows, int ncols, const int64_t* indptr, const int32_t* i
     }
 }
 
+}  // namespace
+#include "pattern_host.cuh"
+namespace {
+
 cudaStream_t st(void* stream) { return (cudaStream_t)stream; }
 
 // Bracket one launch of the profiled kernel with a pair of events on its
@@ -376,6 +389,18 @@ const DevEll<double>& lvM<double>(const Level& l) { return l.M; }
 template <>
 const DevEll<float>& lvM<float>(const Level& l) { return l.Mf; }
 template <class T>
+std::vector<Pat<T>>& patDn(pycfd_solver* s);
+template <>
+std::vector<Pat<double>>& patDn<double>(pycfd_solver* s) { return s->pdn; }
+template <>
+std::vector<Pat<float>>& patDn<float>(pycfd_solver* s) { return s->pdnf; }
+template <class T>
+std::vector<Pat<T>>& patUp(pycfd_solver* s);
+template <>
+std::vector<Pat<double>>& patUp<double>(pycfd_solver* s) { return s->pup; }
+template <>
+std::vector<Pat<float>>& patUp<float>(pycfd_solver* s) { return s->pupf; }
+template <class T>
 const T* tailM(pycfd_solver* s);
 template <>
 const double* tailM<double>(pycfd_solver* s) { return s->tail; }
@@ -463,6 +488,33 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
     pdl_launch(s, k_dense<T>, 1, 256, 0, stream, coarseC<T>(s), s->nc, B0.b, z_out);
     CHECK_LAUNCH();
     pdl_launch(s, k_fine_sums<T, 1>, s->cgrid, s->cblock, 0, stream, z_out, s->flags, g, r, s->singular, s->S, s->rb());
+    CHECK_LAUNCH();
+    return 0;
+  }
+  if (!patDn<T>(s).empty()) {
+    const int tl = s->tail_level;
+    auto product = [&](const Pat<T>& E, const T* s1, const T* s2, T* y, bool from_r) -> int {
+      const int L = pat_parts1(E.n, E.K + E.K2, s->pat_threads);
+      const int grid = (E.n + 256 / L - 1) / (256 / L);
+      if (from_r)
+        pdl_launch(s, k_pat<T, true>, grid, 256, 0, stream, E, L, s1, s2, (const double*)s->S, s->singular, y);
+      else
+        pdl_launch(s, k_pat<T, false>, grid, 256, 0, stream, E, L, s1, s2, (const double*)s->S, s->singular, y);
+      CHECK_LAUNCH();
+      return 0;
+    };
+    for (int l = 1; l <= tl; ++l)
+      TRY(product(patDn<T>(s)[l], l == 1 ? r : lvB<T>(s->lv[l - 1]).b, (const T*)nullptr, lvB<T>(s->lv[l]).b, l == 1));
+    LevelBuf<T>& Bt = lvB<T>(s->lv[tl]);
+    pdl_launch(s, k_tail<T>, (s->lv[tl].n + kTailRowsPerBlock - 1) / kTailRowsPerBlock, 256, 0, stream, tailM<T>(s),
+               s->lv[tl].n, (const T*)Bt.b, Bt.xa);
+    CHECK_LAUNCH();
+    for (int l = tl - 1; l >= 1; --l)
+      TRY(product(patUp<T>(s)[l], lvB<T>(s->lv[l + 1]).xa, lvB<T>(s->lv[l]).b, lvB<T>(s->lv[l]).xa, false));
+    prof_mark(s, 2, stream);
+    pdl_launch(s, k_pat_up0<T>, grid_for(s->ncell(), 256, kMaxRedBlocks), 256, 0, stream, patUp<T>(s)[0],
+               (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, g, s->singular, s->S, z_out, s->rb());
+    prof_mark(s, 2, stream);
     CHECK_LAUNCH();
     return 0;
   }
@@ -919,6 +971,38 @@ int solve_persistent(pycfd_solver* s, double* x, bool has_x0, cudaStream_t strea
   return 0;
 }
 
+// The V-cycle of an MG-PCG solver as pattern products, where its form allows: one sweep
+// per level, a dense tail, fused restrictions asked for, no other form of the coarse
+// levels, a uniform mesh (on a stretched one every row differs) and few enough patterns.
+// They then take the place of the level operators, which are not uploaded.
+bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
+  *rc = 0;
+  const int t = d->tail_level;
+  if (s->solver_kind != PCFD_SOLVER_MGCG || s->mg_sweeps != 1 || t < 1 || t >= d->n_levels - 1 || !d->tail_operator ||
+      s->met || d->coarse_cluster_rows > 0 || d->persistent_solve)
+    return false;
+  for (int l = 1; l <= t; ++l)
+    if (!d->levels[l].m_indptr) return false;
+  PatCycle<double> cd;
+  PatCycle<float> cf;
+  std::vector<std::function<bool()>> tasks;
+  if (!pat_tasks<double>(d->levels, t, false, s->hflags.data(), &cd, &tasks)) return false;
+  if (s->precision == PCFD_MIXED && !pat_tasks<float>(d->levels, t, false, s->hflags.data(), &cf, &tasks)) return false;
+  if (!run_tasks(tasks)) return false;
+  auto keep = [&](auto& c, auto& dn, auto& up) -> int {
+    dn.resize(t + 1);
+    up.resize(t + 1);
+    for (int l = 0; l < t; ++l) {
+      TRY(pat_upload(s, c.dn[l + 1], &dn[l + 1]));
+      TRY(pat_upload(s, c.up[l], &up[l]));
+    }
+    return 0;
+  };
+  if ((*rc = keep(cd, s->pdn, s->pup))) return false;
+  if (s->precision == PCFD_MIXED && (*rc = keep(cf, s->pdnf, s->pupf))) return false;
+  return true;
+}
+
 // ---- Jacobi-CG as one cluster launch ----------------------------------------
 using ClKernel = void (*)(ClSolve);
 ClKernel cl_kernel(int cells) {
@@ -1252,7 +1336,11 @@ int pycfd_solver_destroy(pycfd_solver* s) {
   return 0;
 }
 
-int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) {
+}  // extern "C"
+
+// member: the solver carries one problem of a batch (geometry, masks, vectors); the batch
+// runs its solves.
+static int solver_create(const pycfd_solver_desc* d, bool member, pycfd_solver** out) {
   if (!d || !out) return fail(PCFD_E_ARG, "null descriptor");
   if (d->nx < 4 || d->ny < 4) return fail(PCFD_E_ARG, "mesh must be at least 4x4 cells");
   if (d->solver_kind < PCFD_SOLVER_CG || d->solver_kind > PCFD_SOLVER_MGCG)
@@ -1322,6 +1410,7 @@ int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) {
   {
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    s->pat_threads = (long)nsm * 2048;
     // default: eight 256-thread blocks per SM (measured best of 4..12 on the 512^2 vortex;
     // with the ELL kernels' <= 48 registers five are resident, the rest follow as they end)
     s->ell_budget = d->ell_thread_budget ? (long)d->ell_thread_budget : (long)nsm * 8 * 256;
@@ -1371,6 +1460,7 @@ int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) {
   }
   int rc;
   if ((rc = upload(s, &s->flags, flags.data(), n))) return bail(rc);
+  s->hflags = std::move(flags);
   if ((rc = upload(s, &s->solid, solid.data(), n))) return bail(rc);
 
   // ---- mask face lists (pycfd/core/solver.py:62-79, :285-296) ----
@@ -1469,6 +1559,8 @@ int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) {
     if (d->n_levels < 1 || !d->levels || !d->coarsest_inverse)
       return bail(fail(PCFD_E_ARG, "multigrid solver needs a hierarchy"));
     if (d->levels[0].n != n) return bail(fail(PCFD_E_ARG, "level 0 must have nx*ny unknowns"));
+    const bool pats = pattern_cycle(s, d, &rc);
+    if (rc) return bail(rc);
     s->lv.resize(d->n_levels);
     for (int l = 0; l < d->n_levels; ++l) {
       const pycfd_mg_level& in = d->levels[l];
@@ -1482,7 +1574,7 @@ int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) {
           (rc = dalloc(s, &L.d.res, L.n)) || (rc = dalloc(s, &L.f.b, L.n)) || (rc = dalloc(s, &L.f.xa, L.n)) ||
           (rc = dalloc(s, &L.f.xb, L.n)) || (rc = dalloc(s, &L.f.res, L.n)))
         return bail(rc);
-      if (l >= 1) {
+      if (l >= 1 && !pats) {
         const pycfd_mg_level& up = d->levels[l - 1];
         if (!coarsest) {
           if (!in.a_indptr || !in.weighted_dinv) return bail(fail(PCFD_E_ARG, "level %d lacks A", l));
@@ -1589,16 +1681,20 @@ int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) {
     if ((rc = dalloc(s, &s->pbar, 64)) || (rc = dalloc(s, &s->ppart, (size_t)s->persistent * 2 * kPMaxNV)))
       return bail(rc);
   }
-  if ((rc = cluster_shape(s))) return bail(rc);
   if (s->precision == PCFD_MIXED) {
     if ((rc = dalloc(s, &s->r32, n)) || (rc = dalloc(s, &s->x32, n)) || (rc = dalloc(s, &s->pa32, n)) ||
         (rc = dalloc(s, &s->pb32, n)) || (rc = dalloc(s, &s->q32, n)) || (rc = dalloc(s, &s->z32, n)))
       return bail(rc);
   }
+  if (!member && (rc = cluster_shape(s))) return bail(rc);
   if (cudaDeviceSynchronize() != cudaSuccess) return bail(fail(PCFD_E_CUDA, "setup failed"));
   *out = s;
   return 0;
 }
+
+extern "C" {
+
+int pycfd_solver_create(const pycfd_solver_desc* d, pycfd_solver** out) { return solver_create(d, false, out); }
 
 int pycfd_solver_momentum_rhs(pycfd_solver* s, const double* u, const double* v, double blend, double* rhs_u,
                               double* rhs_v, void* stream) {
