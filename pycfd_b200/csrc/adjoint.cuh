@@ -40,13 +40,13 @@ __global__ void k_adj_predictor(AdjGeo G, const double* __restrict__ U, const do
     if (e < nu) {
       const int m = (int)(e / (n + 2)), j = (int)(e % (n + 2));
       double val = U[e];
-      if (G.u_solv(m, j)) val = val + rmul(dt, rhs_u_at(U, V, m, j, n, G.h, G.h, G.nu, 0.0, 0.0));
+      if (G.u_solv(m, j)) val = val + rmul(dt, rhs_u_at(U, V, m, j, n, RhsK(G.h, G.h, 0.0), G.nu, 0.0, 0.0));
       us[e] = val;
     } else {
       const long f = e - nu;
       const int i = (int)(f / (n + 3)), k = (int)(f % (n + 3));
       double val = V[f];
-      if (G.v_solv(i, k)) val = val + rmul(dt, rhs_v_at(U, V, i, k, n, G.h, G.h, G.nu, 0.0, 0.0));
+      if (G.v_solv(i, k)) val = val + rmul(dt, rhs_v_at(U, V, i, k, n, RhsK(G.h, G.h, 0.0), G.nu, 0.0, 0.0));
       vs[f] = val;
     }
   }

@@ -713,6 +713,7 @@ B_STRIP_KERNEL k_b_predictor(const BProb<T>* __restrict__ probs,
   double* __restrict__ us = b_arr_u(P, dst);
   double* __restrict__ vs = b_arr_v(P, dst);
   const double dt = P.S[S_DT], blend = P.S[S_BLEND];
+  const RhsK kc(g.dx, g.dy, blend);
   const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
   const int segs = (ny + 3 + kBPredCols - 1) / kBPredCols;
   const int items = segs * ((nx + 3 + RS - 1) / RS);
@@ -741,15 +742,15 @@ B_STRIP_KERNEL k_b_predictor(const BProb<T>* __restrict__ probs,
       if (out && ju && m < nx + 3) {
         double val = U[q + 1];
         if (m >= g.u_lo && m < g.u_hi && j >= 1 && j <= ny)
-          val = val + rmul(dt, rhs_u_core(U[q + 1], U[q + 2], U[q], un, usv, vn0, vn1, V[q], V[q + 1], g.dx,
-                                          g.dy, g.nu, blend, g.fx));
+          val = val + rmul(dt, rhs_u_core(U[q + 1], U[q + 2], U[q], un, usv, vn0, vn1, V[q], V[q + 1], kc, g.nu,
+                                          blend, g.fx));
         us[(long)m * W + j] = val;
       }
       if (out && jv && m < nx + 2) {
         double val = V[q + 1];
         if (m >= 1 && m <= nx && j >= g.v_lo && j < g.v_hi)
-          val = val + rmul(dt, rhs_v_core(V[q + 1], vn1, vsv, V[q + 2], V[q], us2, U[q + 2], usv, U[q + 1],
-                                          g.dx, g.dy, g.nu, blend, g.fy));
+          val = val + rmul(dt, rhs_v_core(V[q + 1], vn1, vsv, V[q + 2], V[q], us2, U[q + 2], usv, U[q + 1], kc,
+                                          g.nu, blend, g.fy));
         vs[(long)m * WV + j] = val;
       }
     }
@@ -2051,6 +2052,7 @@ __global__ void __launch_bounds__(kBThreads, PCFD_BELL_MINB) k_b_ellg(const BPro
 // over a warp.  Per launch on 256 cavities in one engine (us): down onto level 1 60 -> 35,
 // onto 2 30 -> 22; level 1 up 76 (two launches) -> 37, level 2 up 58 -> 27; level 0 with
 // its last sweep 109 (two launches) -> 68.
+constexpr int kPatGroup = 8;    // problems per block of a coarse level at most
 constexpr int kPatPart = 12;    // entries a part of a row takes at least
 constexpr int kPatMaxL = 8;     // parts of a row at most
 inline int pat_parts(int K) {
@@ -2068,20 +2070,14 @@ __device__ __forceinline__ void b_pat_rows(const Pat<T>& E, const T* const (&s1)
   const int rpb = kBThreads / L;
   const int part = (int)threadIdx.x / rpb, rl = (int)threadIdx.x - part * rpb;
   const int row = rb * rpb + rl;
-  const int K = E.K + (TWO ? E.K2 : 0);
-  const int per = (K + L - 1) / L, k0 = part * per, k1 = min(K, k0 + per);
+  const int units = (E.K + (TWO ? E.K2 : 0)) / kPatUnit;
   T acc[GS];
 #pragma unroll
   for (int g = 0; g < GS; ++g) acc[g] = (T)0;
-  if (row < E.n) {
-    const PatEntry<T>* tb = E.tab + (long)E.pid[row] * K;
-    if (k0 < E.K)
-      pat_entries<GS, 0, !TWO>(tb + k0, min(k1, E.K) - k0, pat_base(E, row), s1, sh1, acc);
-    if (TWO && k1 > E.K) {
-      const int q = max(k0, E.K);
-      pat_entries<GS, 0, false>(tb + q, k1 - q, row, s2, sh1, acc);
-    }
-  }
+  if (row < E.n)
+    pat_units<GS>(E, pat_tab(E, row), pat_base(E, row), row, part * units / L, (part + 1) * units / L,
+                  [&](int g, int c) { return TWO ? s1[g][c] : s1[g][c] - sh1[g]; },
+                  [&](int g, int c) { return s2[g][c]; }, acc);
   if (L == 1) {
     if (row < E.n) {
 #pragma unroll
@@ -2101,6 +2097,8 @@ __device__ __forceinline__ void b_pat_rows(const Pat<T>& E, const T* const (&s1)
   }
 }
 
+// Problems per block (gs <= kPatGroup) change no problem's arithmetic, so the engine picks
+// them by what the launch leaves idle (pat_group in the runtime).
 // The solving members of a block's group, packed to the front; the slots behind them
 // repeat the first member's sources and have no output.
 template <class T, int GS>
@@ -2161,17 +2159,17 @@ template <class T>
 __global__ void __launch_bounds__(kBThreads, sizeof(T) == 4 ? 4 : 3) k_b_down(const BProb<T>* __restrict__ probs,
                                                          const BHier<T>* __restrict__ hiers,
                                                          const int2* __restrict__ map,
-                                                         const int* __restrict__ sprobs, int d, BShared sh) {
+                                                         const int* __restrict__ sprobs, int gs, int d, BShared sh) {
   pdl_begin();   // programmatic dependent launch: the predecessor's results first
-  constexpr int GM = kBGroup;
+  constexpr int GM = kPatGroup;
   const int2 e = map[blockIdx.x];   // (structure, row block x 1024 + group)
   const BHier<T>& H = hiers[e.x];
   __shared__ BPatGroup<T, GM> G;
   const Pat<T> E = H.dn[d];
   const int L = H.ld[d];
   if (threadIdx.x < 32) {
-    const int k = (e.y & 1023) * GM + (int)threadIdx.x;
-    int pi = (int)threadIdx.x < GM && k < H.spn ? sprobs[H.sp0 + k] : -1;
+    const int k = (e.y & 1023) * gs + (int)threadIdx.x;
+    int pi = (int)threadIdx.x < gs && k < H.spn ? sprobs[H.sp0 + k] : -1;
     if (pi >= 0 && !b_solving(sh, pi)) pi = -1;
     const T* a = nullptr;
     T* o = nullptr;
@@ -2202,17 +2200,17 @@ template <class T>
 __global__ void __launch_bounds__(kBThreads, sizeof(T) == 4 ? 4 : 3) k_b_up(const BProb<T>* __restrict__ probs,
                                                        const BHier<T>* __restrict__ hiers,
                                                        const int2* __restrict__ map,
-                                                       const int* __restrict__ sprobs, int d, BShared sh) {
+                                                       const int* __restrict__ sprobs, int gs, int d, BShared sh) {
   pdl_begin();   // programmatic dependent launch: the predecessor's results first
-  constexpr int GM = kBGroup;
+  constexpr int GM = kPatGroup;
   const int2 e = map[blockIdx.x];   // (structure, row block x 1024 + group)
   const BHier<T>& H = hiers[e.x];
   __shared__ BPatGroup<T, GM> G;
   const Pat<T> E = H.up[d];
   const int L = H.lu[d];
   if (threadIdx.x < 32) {
-    const int k = (e.y & 1023) * GM + (int)threadIdx.x;
-    int pi = (int)threadIdx.x < GM && k < H.spn ? sprobs[H.sp0 + k] : -1;
+    const int k = (e.y & 1023) * gs + (int)threadIdx.x;
+    int pi = (int)threadIdx.x < gs && k < H.spn ? sprobs[H.sp0 + k] : -1;
     if (pi >= 0 && !b_solving(sh, pi)) pi = -1;
     const T *a = nullptr, *b = nullptr;
     T* o = nullptr;
@@ -2240,14 +2238,15 @@ __global__ void __launch_bounds__(kBThreads, sizeof(T) == 4 ? 4 : 3) k_b_up(cons
 }
 
 // Level 0: z = Q_0 x_1 + G_0 b_0 (b_0 the projected CG residual), with sum z and r.z per
-// problem.  kUpRounds blocks of 256 rows for kUpGroup problems per block, so that the
-// block's sums (two per member) are closed once for 2048 rows of each problem.
+// problem.  Several rounds of 256 rows for gs <= kUpGroup problems per block, so that the
+// block's sums (two per member) are closed once for 1024 or 2048 rows of each problem.
 constexpr int kUpGroup = 4;
-constexpr int kUpRounds = 8;
+// rounds by rows: 8 from 32768 rows on, 4 below (a structure's own, since they order its sums)
+__host__ __device__ inline int b_up_rounds(int n) { return n >= 32768 ? 8 : 4; }
 template <class T>
 __global__ void __launch_bounds__(kBThreads, 3)
     k_b_up0(const BProb<T>* __restrict__ probs, const BHier<T>* __restrict__ hiers, const int2* __restrict__ map,
-            const int* __restrict__ sprobs, BShared sh) {
+            const int* __restrict__ sprobs, int gs, BShared sh) {
   pdl_begin();   // programmatic dependent launch: the predecessor's results first
   constexpr int GM = kUpGroup;
   const int2 e = map[blockIdx.x];   // (structure, row block x 4096 + group)
@@ -2255,13 +2254,13 @@ __global__ void __launch_bounds__(kBThreads, 3)
   __shared__ BPatGroup<T, GM> G;
   __shared__ unsigned closing;
   const Pat<T> E = H.up[0];
-  const bool usual = E.K == 6 && E.K2 == 5;   // 2 x 2 aggregates of the five-point operator
+  const bool usual = pat_is_65(E);
   const int KT = E.K + E.K2;
   const int rb = e.y >> 12;
   const uint8_t* __restrict__ flags = probs[sprobs[H.sp0]].flags;   // the structure's
   if (threadIdx.x < 32) {
-    const int k = (e.y & 4095) * GM + (int)threadIdx.x;
-    int pi = (int)threadIdx.x < GM && k < H.spn ? sprobs[H.sp0 + k] : -1;
+    const int k = (e.y & 4095) * gs + (int)threadIdx.x;
+    int pi = (int)threadIdx.x < gs && k < H.spn ? sprobs[H.sp0 + k] : -1;
     if (pi >= 0 && !b_solving(sh, pi)) pi = -1;
     const T *a = nullptr, *b = nullptr;
     T* o = nullptr;
@@ -2280,13 +2279,13 @@ __global__ void __launch_bounds__(kBThreads, 3)
   double sum[2 * GM];
 #pragma unroll
   for (int g = 0; g < 2 * GM; ++g) sum[g] = 0.0;
-  const int row1 = min(E.n, (rb + 1) * kUpRounds * kBThreads);
+  const int per = b_up_rounds(E.n) * kBThreads, row1 = min(E.n, (rb + 1) * per);
   b_pat_width<GM>(G.n, [&](auto w) {
     constexpr int GS = decltype(w)::value;
     const T *a[GS], *b[GS];
     T mr[GS];
     b_pat_copy(G, a, b, mr);
-    int row = rb * kUpRounds * kBThreads + (int)threadIdx.x;
+    int row = rb * per + (int)threadIdx.x;
     int pid = row < row1 ? E.pid[row] : 0;
     uint8_t fl = row < row1 ? flags[row] : 0;
     for (; row < row1; row += kBThreads) {
@@ -2303,13 +2302,10 @@ __global__ void __launch_bounds__(kBThreads, 3)
         acc[g] = (T)0;
         own[g] = b[g][row];
       }
-      if (usual) {
-        pat_entries<GS, 6, false>(tb, 6, pat_base(E, row), a, mr, acc);
-        pat_entries<GS, 5, true>(tb + 6, 5, row, b, mr, acc);
-      } else {
-        pat_entries<GS, 0, false>(tb, E.K, pat_base(E, row), a, mr, acc);
-        pat_entries<GS, 0, true>(tb + E.K, E.K2, row, b, mr, acc);
-      }
+      auto xa = [&](int g, int c) { return a[g][c]; };
+      auto xb = [&](int g, int c) { return b[g][c] - mr[g]; };
+      if (usual) pat_whole<true, GS>(E, tb, row, xa, xb, acc);
+      else pat_whole<false, GS>(E, tb, row, xa, xb, acc);
 #pragma unroll
       for (int g = 0; g < GS; ++g) {
         if (T* o = G.out[g]) o[row] = acc[g];

@@ -26,6 +26,8 @@ struct pycfd_batch {
   int fused_from = 1;                      // first level restricted by the fused product (1 or 2)
   int ell_group = kBGroup;                 // problems per block of the coarse-level launches (1 or kBGroup)
   int pats = 0;                            // the cycle above the tails as pattern products
+  int pat_group = kPatGroup;               // problems per block of their coarse-level launches,
+  int up_group = kUpGroup;                 // and of the level-0 up product
   BMapHost map0;                           // level-0 up product: (structure, row block x 4096 + group of kUpGroup)
   int stencil_req = 0;                     // level-0 transfers as stencils, as asked
   int stencil = 0;                         // ... and in force (fused down sweep from the fine level)
@@ -262,7 +264,8 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
       P.h_tiles_j = (s->g.ny + kBHaloTC - 1) / kBHaloTC;
       P.h_tiles = ((s->g.nx + tr - 1) / tr) * P.h_tiles_j;
     }
-    P.u_chunks = (s->g.nx * s->g.ny + kUpRounds * kBThreads - 1) / (kUpRounds * kBThreads);
+    const int up_rows = b_up_rounds(s->g.nx * s->g.ny) * kBThreads;
+    P.u_chunks = (s->g.nx * s->g.ny + up_rows - 1) / up_rows;
     P.red_base = red_rows;
     red_rows += std::max({P.chunks, P.s_chunks, P.v_chunks, P.h_tiles, P.u_chunks});
     P.flags = s->flags;
@@ -371,6 +374,33 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     if (!hh[h].agg2)
       return fail(PCFD_E_UNSUPPORTED, "stencil transfers: structure %d's level 1 is not the 2 x 2 aggregation",
                   (int)h);
+  // Problems per block of the pattern products: as many as leave every SM a block (at
+  // level 1, and at level 0), at most 8 and 4 (FP32) or 4 and 2 (FP64, whose accumulators
+  // take twice the registers).  Against half of each: 256 cavities mixed 10.2 / 10.5 ms per
+  // step, 24 small ones 3.4 / 2.9, 64 in FP64 4.4 / 4.0.
+  if (B->pats) {
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    auto pick = [&](int most, int limit, auto rows) {   // limit: groups per structure the block map can name
+      auto groups = [&](size_t h, int gs) { return (hh[h].spn + gs - 1) / gs; };
+      int gs = most;
+      for (; gs > 1; gs /= 2) {
+        long blocks = 0, widest = 0;
+        for (size_t h = 0; h < leaders.size(); ++h) {
+          blocks += (long)rows(h) * groups(h, gs);
+          widest = std::max<long>(widest, groups(h, gs / 2));
+        }
+        if (blocks >= nsm || widest > limit) break;
+      }
+      return gs;
+    };
+    const int half = sizeof(T) == 4 ? 1 : 2;
+    B->pat_group = pick(kPatGroup / half, 1024, [&](size_t h) {
+      const int rpb = kBThreads / hh[h].ld[1];
+      return (keep[h][1].n + rpb - 1) / rpb;
+    });
+    B->up_group = pick(kUpGroup / half, 4096, [&](size_t h) { return pr[leaders[h]].u_chunks; });
+  }
   B->mapA.assign(B->depth, BMapHost{});
   B->mapR.assign(B->depth, BMapHost{});
   B->mapP.assign(B->depth, BMapHost{});
@@ -380,7 +410,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     std::vector<int2> ma, mr, mp, mc;
     for (size_t h = 0; h < leaders.size(); ++h) {
       const BHier<T>& H = hh[h];
-      const int gs = B->ell_group;
+      const int gs = B->pats ? B->pat_group : B->ell_group;
       const int grps = (H.spn + gs - 1) / gs;
       if (grps > 1024) return fail(PCFD_E_UNSUPPORTED, "at most %d problems share a structure", 1024 * gs);
       if (H.tail_level == d && H.tail_n > 0) {
@@ -393,8 +423,8 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
         if (d > H.tail_level) continue;
         const int nrow = d == 0 ? pr[leaders[h]].g.nx * pr[leaders[h]].g.ny : keep[h][d].n;
         if (d == 0) {
-          const int g4 = (H.spn + kUpGroup - 1) / kUpGroup;
-          for (int rb = 0; rb * kUpRounds * kBThreads < nrow; ++rb)
+          const int g4 = (H.spn + B->up_group - 1) / B->up_group;
+          for (int rb = 0; rb < pr[leaders[h]].u_chunks; ++rb)
             for (int g = 0; g < g4; ++g) m0.push_back(make_int2((int)h, rb * 4096 + g));
           continue;
         }
@@ -571,17 +601,18 @@ int b_vcycle(pycfd_batch* B, cudaStream_t st) {
     for (int d = 1; d < D; ++d)
       if (B->mapR[d].n)
         BLAUNCH(k_b_down<T>, B->mapR[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapR[d].e, B->sprobs,
-                d, B->sh);
+                B->pat_group, d, B->sh);
     b_prof(B, 4, st);
     TRY(b_tails<T>(B, st));
     b_prof(B, 4, st);
     for (int d = D - 1; d >= 1; --d)
       if (B->mapA[d].n)
-        BLAUNCH(k_b_up<T>, B->mapA[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapA[d].e, B->sprobs, d,
-                B->sh);
+        BLAUNCH(k_b_up<T>, B->mapA[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapA[d].e, B->sprobs,
+                B->pat_group, d, B->sh);
     b_prof(B, 4, st);
     b_prof(B, 2, st);
-    BLAUNCH(k_b_up0<T>, B->map0.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->map0.e, B->sprobs, B->sh);
+    BLAUNCH(k_b_up0<T>, B->map0.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->map0.e, B->sprobs,
+            B->up_group, B->sh);
     b_prof(B, 2, st);
     return 0;
   }

@@ -202,25 +202,28 @@ constexpr int kTailRowsPerBlock = 256 / 32 / kTailWarps;
 template <class T>
 __global__ void __launch_bounds__(256) k_tail(const T* __restrict__ M, int n, const T* __restrict__ b,
                                               T* __restrict__ x) {
-  pdl_begin();
   __shared__ double part[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * kTailRowsPerBlock + warp / kTailWarps;
   const int w = warp % kTailWarps;
+  constexpr int stride = 32 * kTailWarps;
+  const T* m = M + (long)(row < n ? row : 0) * n;
+  T mm[8];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) mm[u] = k0 + u * stride < n ? __ldg(m + k0 + u * stride) : (T)0;
+  };
+  load(w * 32 + lane);   // no kernel writes M: ahead of the wait
+  pdl_begin();
   double acc = 0.0;
   if (row < n) {
-    const T* m = M + (long)row * n;
-    constexpr int stride = 32 * kTailWarps;
     for (int k0 = w * 32 + lane; k0 < n; k0 += 8 * stride) {
-      T mm[8], bb[8];
+      T bb[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = k0 + u * stride;
-        mm[u] = k < n ? __ldg(m + k) : (T)0;
-        bb[u] = k < n ? b[k] : (T)0;
-      }
+      for (int u = 0; u < 8; ++u) bb[u] = k0 + u * stride < n ? b[k0 + u * stride] : (T)0;
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc += (double)mm[u] * (double)bb[u];
+      if (k0 + 8 * stride < n) load(k0 + 8 * stride);
     }
   }
   acc = warp_sum(acc);
@@ -307,118 +310,119 @@ __global__ void k_ell_prolong0_wb(Ell<T> P, B bf, const uint8_t* __restrict__ fl
 }
 
 // ---- pattern products of one problem -------------------------------------------
-// Down and up products of the cycle above the dense tail (pattern.cuh), 256 / L rows per
-// block, a row's entries split over L parts of the block whose sums are added in part
-// order.  A single problem's levels are short, so the launch is bound by its chain of
-// dependent loads: the pattern and its first entries (tables no kernel writes) are read
-// before the wait for the predecessor, and one round of gathers is left behind it.
-constexpr int kPatChunk = 8;        // entries gathered together
+// Down and up products of the cycle above the dense tail (pattern.cuh); products and sums
+// in double, whatever the storage type.  A block takes a tile of 32 rows along y by
+// 8 / L along x (from L = 16 on, 256 / L rows along y), so that the values it gathers are
+// shared along both axes in L1, and splits the entries of the short levels over L parts of
+// the block, their sums added in part order.  Four blocks of 64 registers per SM: 5 and 8
+// (fewer gathers in flight each) step the 2048x1024 cylinder in 11.2 and 11.8 ms against
+// 10.2.
+#ifndef PCFD_PAT_MINB
+#define PCFD_PAT_MINB 4
+#endif
 constexpr int kPatMaxParts = 32;
-// Parts per row: about three entries each, within the resident threads of the GPU.
-inline int pat_parts1(int n, int K, long threads) {
+// Rows along y of a tile.
+__host__ __device__ inline int pat_tile_j(int L) { return L <= 8 ? 32 : 256 / L; }
+struct PatLaunch {
   int L = 1;
-  while (L < kPatMaxParts && K >= 6 * L && (long)n * L * 2 <= threads) L *= 2;
-  return L;
+  dim3 grid;
+};
+// Parts: about two units each, within the resident threads of the GPU.
+template <class T>
+inline PatLaunch pat_launch(const Pat<T>& E, long threads, bool parts) {
+  PatLaunch p;
+  const int K = E.K + E.K2, rx = E.n / E.ny_r;
+  while (parts && p.L < kPatMaxParts && K >= 2 * kPatUnit * p.L && (long)E.n * p.L * 2 <= threads) p.L *= 2;
+  const int tj = pat_tile_j(p.L), ti = 256 / p.L / tj;
+  p.grid = dim3((E.ny_r + tj - 1) / tj, (rx + ti - 1) / ti);
+  return p;
+}
+template <class T>
+__device__ __forceinline__ int pat_base_ij(const Pat<T>& E, int i, int j) {
+  return E.base == PB_COARSER ? (i >> (E.fx - 1)) * E.ny_c + (j >> (E.fy - 1))
+         : E.base == PB_FINER ? (i << (E.fx - 1)) * E.ny_c + (j << (E.fy - 1))
+                              : i * E.ny_r + j;
 }
 
-// Sum of row `row` over entries [k0, k1): E's first source from its base, the second
-// from the row; `begin` runs between the first table reads and the first gather.
-template <class T, class Begin, class X1, class X2>
-__device__ __forceinline__ double pat_sum(const Pat<T>& E, int row, int k0, int k1, Begin begin, X1 x1, X2 x2) {
-  const bool ok = row < E.n && k0 < k1;
-  const int K = E.K + E.K2;
-  const int base = ok ? pat_base(E, row) : 0;
-  const PatEntry<T>* tb = E.tab + (ok ? (long)E.pid[row] * K : 0);
-  int at[kPatChunk];
-  T val[kPatChunk];
-  auto load = [&](int k) {
-#pragma unroll
-    for (int u = 0; u < kPatChunk; ++u) {
-      at[u] = 0;
-      val[u] = (T)0;
-      if (k + u < k1) {
-        pat_load(tb + k + u, &at[u], &val[u]);
-        at[u] += k + u < E.K ? base : row;
-      }
-    }
-  };
-  if (ok) load(k0);
-  begin();
-  double acc = 0.0;
-  if (!ok) return acc;
-  for (int k = k0;;) {
-    double x[kPatChunk];
-#pragma unroll
-    for (int u = 0; u < kPatChunk; ++u) x[u] = k + u < k1 ? (k + u < E.K ? x1(at[u]) : x2(at[u])) : 0.0;
-#pragma unroll
-    for (int u = 0; u < kPatChunk; ++u) acc += (double)val[u] * x[u];
-    k += kPatChunk;
-    if (k >= k1) return acc;
-    load(k);
-  }
-}
-
-// y = E x1 (+ second source x2): FROM_R: the first source of a down product is the CG
-// residual less its fluid mean.
+// y = E s1 (+ second source s2).  FROM_R: the source of a down product is the CG residual
+// less its fluid mean.
 template <class T, bool FROM_R>
-__global__ void __launch_bounds__(256) k_pat(Pat<T> E, int L, const T* __restrict__ s1, const T* __restrict__ s2,
-                                             const double* __restrict__ S, int singular, T* __restrict__ y) {
-  const int rpb = 256 / L;
+__global__ void __launch_bounds__(256, PCFD_PAT_MINB)
+    k_pat(Pat<T> E, int L, const T* __restrict__ s1, const T* __restrict__ s2, const double* __restrict__ S,
+          int singular, T* __restrict__ y) {
+  const int tj = pat_tile_j(L), rpb = 256 / L, ti = rpb / tj;
   const int part = (int)threadIdx.x / rpb, rl = (int)threadIdx.x - part * rpb;
-  const int row = (int)blockIdx.x * rpb + rl;
-  const int K = E.K + E.K2, per = (K + L - 1) / L, k0 = part * per, k1 = min(K, k0 + per);
-  double mean = 0.0;
-  const double acc = pat_sum(
-      E, row, k0, k1,
-      [&]() {
-        pdl_begin();
-        if (FROM_R && singular) mean = S[S_MEAN_R];
-      },
-      [&](int c) { return FROM_R ? (double)s1[c] - mean : (double)s1[c]; }, [&](int c) { return (double)s2[c]; });
+  const int i = (int)blockIdx.y * ti + rl / tj, j = (int)blockIdx.x * tj + rl % tj;
+  const int row = i * E.ny_r + j;
+  const bool ok = j < E.ny_r && row < E.n;
+  // the tables, which no kernel writes, ahead of the wait for the predecessor
+  const PatEntry<T>* tb = pat_tab(E, ok ? row : 0);
+  const int units = (E.K + E.K2) / kPatUnit, q0 = part * units / L, q1 = (part + 1) * units / L;
+  pdl_begin();
+  const double mean = FROM_R && singular ? S[S_MEAN_R] : 0.0;
+  double acc[1] = {0.0};
+  if (ok)
+    pat_units<1>(E, tb, pat_base_ij(E, i, j), row, q0, q1,
+                 [&](int, int c) { return FROM_R ? (double)s1[c] - mean : (double)s1[c]; },
+                 [&](int, int c) { return (double)s2[c]; }, acc);
   if (L == 1) {
-    if (row < E.n) y[row] = (T)acc;
+    if (ok) y[row] = (T)acc[0];
     return;
   }
   __shared__ double red[256];
-  red[threadIdx.x] = acc;
+  red[threadIdx.x] = acc[0];
   __syncthreads();
-  if (part == 0 && row < E.n) {
-    double t = acc;
+  if (part == 0 && ok) {
+    double t = acc[0];
     for (int q = 1; q < L; ++q) t += red[q * rpb + rl];
     y[row] = (T)t;
   }
 }
 
 // Level 0: z = Q_0 x_1 + G_0 b_0 (b_0 the projected CG residual) with sum z and r.z for
-// the projected z and rho, one row per thread.
-template <class T>
-__global__ void __launch_bounds__(256) k_pat_up0(Pat<T> E, const T* __restrict__ x1, const T* __restrict__ r,
-                                                 const uint8_t* __restrict__ flags, Geo g, int singular,
-                                                 double* __restrict__ S, T* __restrict__ z, RedBuf rb) {
-  const int K = E.K + E.K2;
+// the projected z and rho; a block walks `rounds` tiles along x.
+template <class T, bool F65>
+__global__ void __launch_bounds__(256, PCFD_PAT_MINB)
+    k_pat_up0(Pat<T> E, int rounds, const T* __restrict__ x1, const T* __restrict__ r,
+              const uint8_t* __restrict__ flags, Geo g, int singular, double* __restrict__ S, T* __restrict__ z,
+              RedBuf rb) {
+  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
+  const int j = (int)blockIdx.x * 32 + lane, nx = E.n / E.ny_r;
+  const int i1 = min(nx, ((int)blockIdx.y + 1) * rounds * 8);
+  int i = (int)blockIdx.y * rounds * 8 + warp;
+  bool ok = j < E.ny_r && i < i1;
+  const PatEntry<T>* tb = pat_tab(E, ok ? i * E.ny_r + j : 0);
+  uint8_t f = ok ? flags[i * E.ny_r + j] : 0;
+  pdl_begin();
+  const double mean = singular ? S[S_MEAN_R] : 0.0;
   double acc[2] = {0, 0};
-  double mean = 0.0;
-  bool waited = false;
-  for (int row0 = (int)blockIdx.x * 256; row0 < E.n; row0 += (int)gridDim.x * 256) {
-    const int row = row0 + (int)threadIdx.x;
-    const uint8_t f = row < E.n ? flags[row] : 0;
-    const double v = pat_sum(
-        E, row, 0, K,
-        [&]() {
-          if (waited) return;
-          pdl_begin();
-          waited = true;
-          if (singular) mean = S[S_MEAN_R];
-        },
-        [&](int c) { return (double)x1[c]; }, [&](int c) { return (double)r[c] - mean; });
-    if (row < E.n) {
-      const double zn = (double)(T)v;
-      z[row] = (T)zn;
-      if (f & F_SOLV) {
-        acc[0] += zn;
-        acc[1] += (double)r[row] * zn;
-      }
+  while (ok) {
+    const int row = i * E.ny_r + j;
+    const PatEntry<T>* tc = tb;
+    const uint8_t fc = f;
+    ok = i + 8 < i1;
+    if (ok) {   // the next row's pattern, ahead of its use
+      tb = pat_tab(E, row + 8 * E.ny_r);
+      f = flags[row + 8 * E.ny_r];
     }
+    const double own = (double)r[row];
+    double v[1] = {0.0};
+    auto xa = [&](int, int c) { return (double)x1[c]; };
+    auto xb = [&](int, int c) { return (double)r[c] - mean; };
+    const int base = pat_base_ij(E, i, j);
+    if constexpr (F65) {
+      pat_batch<6, 1>(tc, base, xa, v);
+      pat_batch<5, 1>(tc + 6, row, xb, v);
+    } else {
+      pat_units<1>(E, tc, base, row, 0, (E.K + E.K2) / kPatUnit, xa, xb, v);
+    }
+    const double zn = (double)(T)v[0];
+    z[row] = (T)zn;
+    if (fc & F_SOLV) {
+      acc[0] += zn;
+      acc[1] += own * zn;
+    }
+    i += 8;
   }
   grid_reduce<2>(acc, rb, [&](double* t) {
     const double m = (singular && g.n_fluid) ? t[0] / g.n_fluid : 0.0;

@@ -46,7 +46,9 @@ __device__ __forceinline__ void pat_load(const PatEntry<double>* e, int* off, do
 enum PatBase { PB_SAME = 0, PB_COARSER = 1, PB_FINER = 2 };
 
 // An operator of one source (K2 = 0), or of two: K entries on the first from its base
-// index, then K2 on the second, a vector on the rows' own grid.
+// index, then K2 on the second, a vector on the rows' own grid.  Both counts are padded to
+// units of four entries (kPatUnit), so that no entry needs a test of its own -- except the
+// level-0 up product of 2 x 2 aggregates, whose 6 + 5 entries have code of their own.
 template <class T>
 struct Pat {
   const uint16_t* pid;        // pattern of each row
@@ -54,50 +56,91 @@ struct Pat {
   int n, K, K2;               // rows, entries per pattern
   int base, ny_r, ny_c;       // PatBase; columns (y cells) of the row and the source grid
   int fx, fy;                 // coarsening factors between them (1 or 2)
+  unsigned inv;               // ceil(2^32 / ny_r): rows are divided by a multiplication
 };
+constexpr int kPatUnit = 4;
 
 template <class T>
 __host__ __device__ __forceinline__ int pat_base(const Pat<T>& E, int row) {
   if (E.base == PB_SAME) return row;
-  const int i = row / E.ny_r, j = row - i * E.ny_r;
+#ifdef __CUDA_ARCH__
+  int i = (int)__umulhi((unsigned)row, E.inv);   // the quotient, or one off
+#else
+  int i = (int)(((unsigned long long)(unsigned)row * E.inv) >> 32);
+#endif
+  int j = row - i * E.ny_r;
+  if (j < 0) {
+    --i;
+    j += E.ny_r;
+  } else if (j >= E.ny_r) {   // ny_r = 1, whose inverse does not fit
+    ++i;
+    j -= E.ny_r;
+  }
   return E.base == PB_COARSER ? (i >> (E.fx - 1)) * E.ny_c + (j >> (E.fy - 1))
                               : (i << (E.fx - 1)) * E.ny_c + (j << (E.fy - 1));
 }
-
-// Entries whose gathers are in flight together: 16 values over the GS members.
-template <class T, int GS>
-__host__ __device__ constexpr int pat_unroll() {
-  constexpr int u = 16 / GS;
-  return u < 2 ? 2 : u > 8 ? 8 : u;
+template <class T>
+__device__ __forceinline__ const PatEntry<T>* pat_tab(const Pat<T>& E, int row) {
+  return E.tab + (long)__ldg(E.pid + row) * (E.K + E.K2);
 }
 
-// acc[g] += sum over `count` entries tb[0 ..] applied to the GS vectors src from index
-// base.  Every member's pointer is valid (an absent one repeats another's), so that no
-// branch separates the members' gathers.  shift: subtracted from every gathered value
-// (the mean of a projected residual).  KC > 0: the count, known when compiling.
-template <int GS, int KC, bool SHIFT, class T>
-__device__ __forceinline__ void pat_entries(const PatEntry<T>* tb, int count, int base, const T* const (&src)[GS],
-                                            const T (&shift)[GS], T (&acc)[GS]) {
-  constexpr int U = KC > 0 ? KC : pat_unroll<T, GS>();
-  if (KC > 0) count = KC;
-  for (int k = 0; k < count; k += U) {
-    int at[U];
-    T val[U], x[U][GS];
+// acc[g] += N entries of tb applied to x(g, index), all gathers issued before the sums.
+template <int N, int GS, class T, class A, class X>
+__device__ __forceinline__ void pat_batch(const PatEntry<T>* tb, int base, X x, A (&acc)[GS]) {
+  int at[N];
+  T val[N];
+  A xv[N][GS];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      at[u] = 0;
-      val[u] = (T)0;
-      if (KC > 0 || k + u < count) pat_load(tb + k + u, &at[u], &val[u]);
-      at[u] += base;
+  for (int u = 0; u < N; ++u) pat_load(tb + u, &at[u], &val[u]);
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+#pragma unroll
+    for (int g = 0; g < GS; ++g) xv[u][g] = x(g, base + at[u]);
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+#pragma unroll
+    for (int g = 0; g < GS; ++g) acc[g] += (A)val[u] * xv[u][g];
+}
+
+// Units [q0, q1) of a row (its table at tb): xa(g, index) gathers the first source, xb the
+// second, for GS members.  Up to 16 gathers are in flight together.
+template <int GS, class T, class A, class XA, class XB>
+__device__ __forceinline__ void pat_units(const Pat<T>& E, const PatEntry<T>* tb, int base, int row, int q0, int q1,
+                                          XA xa, XB xb, A (&acc)[GS]) {
+  const int qa = min(q1, E.K / kPatUnit);
+  int q = q0;
+  if constexpr (GS <= 2) {
+    for (; q + 2 <= qa; q += 2) pat_batch<2 * kPatUnit, GS>(tb + q * kPatUnit, base, xa, acc);
+    if (q < qa) pat_batch<kPatUnit, GS>(tb + q++ * kPatUnit, base, xa, acc);
+    for (; q + 2 <= q1; q += 2) pat_batch<2 * kPatUnit, GS>(tb + q * kPatUnit, row, xb, acc);
+    if (q < q1) pat_batch<kPatUnit, GS>(tb + q * kPatUnit, row, xb, acc);
+  } else if constexpr (GS <= 4) {
+    for (; q < qa; ++q) pat_batch<kPatUnit, GS>(tb + q * kPatUnit, base, xa, acc);
+    for (; q < q1; ++q) pat_batch<kPatUnit, GS>(tb + q * kPatUnit, row, xb, acc);
+  } else {
+    for (; q < qa; ++q) {
+      pat_batch<kPatUnit / 2, GS>(tb + q * kPatUnit, base, xa, acc);
+      pat_batch<kPatUnit / 2, GS>(tb + q * kPatUnit + kPatUnit / 2, base, xa, acc);
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int g = 0; g < GS; ++g) x[u][g] = src[g][at[u]];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int g = 0; g < GS; ++g) acc[g] += val[u] * (SHIFT ? x[u][g] - shift[g] : x[u][g]);
+    for (; q < q1; ++q) {
+      pat_batch<kPatUnit / 2, GS>(tb + q * kPatUnit, row, xb, acc);
+      pat_batch<kPatUnit / 2, GS>(tb + q * kPatUnit + kPatUnit / 2, row, xb, acc);
+    }
+  }
+}
+
+// The whole row: the level-0 up product of 2 x 2 aggregates (6 + 5 entries) by code of its
+// own, any other by units.
+template <class T>
+__host__ __device__ __forceinline__ bool pat_is_65(const Pat<T>& E) { return E.K == 6 && E.K2 == 5; }
+template <bool F65, int GS, class T, class A, class XA, class XB>
+__device__ __forceinline__ void pat_whole(const Pat<T>& E, const PatEntry<T>* tb, int row, XA xa, XB xb, A (&acc)[GS]) {
+  const int base = pat_base(E, row);
+  if constexpr (F65) {
+    pat_batch<6, GS>(tb, base, xa, acc);
+    pat_batch<5, GS>(tb + 6, row, xb, acc);
+  } else {
+    pat_units<GS>(E, tb, base, row, 0, (E.K + E.K2) / kPatUnit, xa, xb, acc);
   }
 }
 

@@ -194,6 +194,7 @@ bool pat_shape(Pat<T>* E, int nr, int rx, int ry, int nc, int cx, int cy) {
   if ((long)rx * ry != nr || (long)cx * cy != nc) return false;
   E->n = nr;
   E->ny_r = ry;
+  E->inv = (unsigned)std::min<unsigned long long>(0xffffffffull, ((1ull << 32) + ry - 1) / (unsigned)ry);
   E->ny_c = cy;
   E->fx = E->fy = 1;
   E->base = PB_SAME;
@@ -229,6 +230,10 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
     K = std::max<int>(K, (int)(A.ptr[r + 1] - A.ptr[r]));
     if (B) K2 = std::max<int>(K2, (int)(B->ptr[r + 1] - B->ptr[r]));
   }
+  if (!(K == 6 && K2 == 5)) {   // units of four entries (pattern.cuh)
+    K = (K + kPatUnit - 1) / kPatUnit * kPatUnit;
+    K2 = (K2 + kPatUnit - 1) / kPatUnit * kPatUnit;
+  }
   const int KT = K + K2;
   const size_t most = std::min<size_t>(65535, n > 16384 && !any ? (size_t)n / 4 : (size_t)n);
   E.K = K;
@@ -237,7 +242,7 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
   out->tab.clear();
   std::vector<PatEntry<T>> row(KT);
   std::unordered_multimap<uint64_t, int> seen;
-  int last = -1;
+  int recent[2] = {-1, -1};   // rows along y alternate between two patterns of a coarsened grid
   auto same = [&](int p) {
     const PatEntry<T>* t = &out->tab[(size_t)p * KT];
     for (int k = 0; k < KT; ++k)
@@ -264,7 +269,9 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
     };
     part(A, liveA, pat_base(E, r), 0, K);
     if (B) part(*B, liveB, r, K, K2);
-    int id = last >= 0 && same(last) ? last : -1;
+    int id = -1;
+    for (int q : recent)
+      if (id < 0 && q >= 0 && same(q)) id = q;
     if (id < 0) {
       auto range = seen.equal_range(h);
       for (auto it = range.first; it != range.second && id < 0; ++it)
@@ -277,7 +284,10 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
       out->tab.insert(out->tab.end(), row.begin(), row.end());
     }
     out->pid[r] = (uint16_t)id;
-    last = id;
+    if (id != recent[0]) {
+      recent[1] = recent[0];
+      recent[0] = id;
+    }
   }
   return true;
 }

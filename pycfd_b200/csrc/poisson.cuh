@@ -87,13 +87,17 @@ __global__ void k_rhs_init(double* __restrict__ b, T* __restrict__ x, T* __restr
 
 // p = z + beta p_old with z = r/d (Jacobi) or z = z_raw - mean_z on solvable
 // rows (multigrid; z_raw from the V-cycle), q = A p, and p.q -> alpha.
+// The direction of pass `it` is pa (it even) or pb (it odd), the previous one the other, so
+// no pass copies p and a recorded loop body reads the right one.
 template <class T, int PC>
-__global__ void k_cg_pq(const T* __restrict__ r, const T* __restrict__ zraw,
-                        const T* __restrict__ p_old, T* __restrict__ p_new, T* __restrict__ q,
+__global__ void k_cg_pq(const T* __restrict__ r, const T* __restrict__ zraw, T* pa, T* pb, T* __restrict__ q,
                         const uint8_t* __restrict__ flags, Geo g, double* __restrict__ S,
                         const int* __restrict__ I, RedBuf rb) {
   pdl_begin();
-  const bool first = I[I_IT] == 0;
+  const int it = I[I_IT];
+  const bool first = it == 0;
+  const T* __restrict__ p_old = (it & 1) ? pa : pb;
+  T* __restrict__ p_new = (it & 1) ? pb : pa;
   const double beta = first ? 0.0 : S[S_RHO] / S[S_RHO_PREV];
   const double mz = S[S_MEAN_Z];
   auto pval = [&](int k, int ii, int jj) -> double {
@@ -121,14 +125,12 @@ __global__ void k_cg_pq(const T* __restrict__ r, const T* __restrict__ zraw,
 
 // x += alpha p, r -= alpha q; ||r||^2, r.(r/d), sum_solvable(r); convergence
 // test of the next pass (scipy's top-of-loop ||r|| < atol), iteration count.
-// p_keep != nullptr: also store p there, so a recorded loop body always reads
-// the previous direction from the same buffer.
 template <class T, int PC>
-__global__ void k_cg_xr(T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                        const T* __restrict__ q, T* __restrict__ p_keep,
+__global__ void k_cg_xr(T* __restrict__ x, T* __restrict__ r, const T* pa, const T* pb, const T* __restrict__ q,
                         const uint8_t* __restrict__ flags, Geo g, SolveCfg cfg,
                         double* __restrict__ S, int* __restrict__ I, RedBuf rb, LoopCtl loop) {
   pdl_begin();
+  const T* __restrict__ p = (I[I_IT] & 1) ? pb : pa;
   const double alpha = S[S_ALPHA];
   double acc[3] = {0, 0, 0};
   T pv[kStripRows], xv[kStripRows], rv[kStripRows], qv[kStripRows];
@@ -146,7 +148,6 @@ __global__ void k_cg_xr(T* __restrict__ x, T* __restrict__ r, const T* __restric
         const T pc = pv[u];
         const double xc = (double)xv[u] + alpha * (double)pc;
         const double rc = (double)(T)((double)rv[u] - alpha * (double)qv[u]);
-        if (p_keep) p_keep[c] = pc;
         x[c] = (T)xc;
         r[c] = (T)rc;
         acc[0] += rc * rc;

@@ -2,12 +2,14 @@
 // lists, multigrid upload), launch orchestration of the substep / projection /
 // Poisson solves, and the C ABI declared in include/pycfd_b200.h.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -156,7 +158,8 @@ struct pycfd_solver {
   // the cycle above the tail as pattern products (empty: the ELL operators)
   std::vector<Pat<double>> pdn, pup;
   std::vector<Pat<float>> pdnf, pupf;
-  long pat_threads = 0;         // resident threads a pattern product spreads its rows over
+  long pat_threads = 0;         // resident threads a pattern product spreads its rows over,
+  int pat_blocks = 1;           // and the blocks they make
   long ell_budget = 0;          // resident threads a per-phase ELL pass may use (< 0: storage lanes)
   int ell_blocks = kWaveBlocks; // grid cap of the per-phase ELL kernels
   double* tail = nullptr;
@@ -199,6 +202,18 @@ struct pycfd_solver {
     DtControl ctl;
   };
   std::vector<GraphEntry> graphs;
+  // recorded solves of the calls that are not recorded whole (solve_rhs)
+  struct SolveGraph {
+    double* x;
+    bool has_x0;
+    cudaGraph_t graph;
+    cudaGraphExec_t exec;
+    long long fixed, body;      // launches outside and inside the iteration loop
+  };
+  std::vector<SolveGraph> solve_graphs;
+  int host_solves = 0;          // solves run with the loop on the host so far
+  long long body_launches = 0;  // launches of the loop body recorded last
+  long long replay_body = 0;    // ... of the replays whose iterations are not counted yet
 
   dim3 cgrid, cblock;   // 2D launch over the fine cells
   RedBuf rb() const { return RedBuf{partials, counter}; }
@@ -494,12 +509,9 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
   if (!patDn<T>(s).empty()) {
     const int tl = s->tail_level;
     auto product = [&](const Pat<T>& E, const T* s1, const T* s2, T* y, bool from_r) -> int {
-      const int L = pat_parts1(E.n, E.K + E.K2, s->pat_threads);
-      const int grid = (E.n + 256 / L - 1) / (256 / L);
-      if (from_r)
-        pdl_launch(s, k_pat<T, true>, grid, 256, 0, stream, E, L, s1, s2, (const double*)s->S, s->singular, y);
-      else
-        pdl_launch(s, k_pat<T, false>, grid, 256, 0, stream, E, L, s1, s2, (const double*)s->S, s->singular, y);
+      const PatLaunch q = pat_launch(E, s->pat_threads, true);
+      pdl_launch(s, from_r ? k_pat<T, true> : k_pat<T, false>, q.grid, 256, 0, stream, E, q.L, s1, s2,
+                 (const double*)s->S, s->singular, y);
       CHECK_LAUNCH();
       return 0;
     };
@@ -512,8 +524,15 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
     for (int l = tl - 1; l >= 1; --l)
       TRY(product(patUp<T>(s)[l], lvB<T>(s->lv[l + 1]).xa, lvB<T>(s->lv[l]).b, lvB<T>(s->lv[l]).xa, false));
     prof_mark(s, 2, stream);
-    pdl_launch(s, k_pat_up0<T>, grid_for(s->ncell(), 256, kMaxRedBlocks), 256, 0, stream, patUp<T>(s)[0],
-               (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, g, s->singular, s->S, z_out, s->rb());
+    {
+      const Pat<T>& E = patUp<T>(s)[0];
+      const PatLaunch q = pat_launch(E, s->pat_threads, false);
+      const long tiles = (long)q.grid.x * q.grid.y;
+      const int rounds = (int)((tiles + s->pat_blocks - 1) / s->pat_blocks);   // one wave of blocks
+      const dim3 grid(q.grid.x, (q.grid.y + rounds - 1) / rounds);
+      pdl_launch(s, pat_is_65(E) ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds,
+                 (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, g, s->singular, s->S, z_out, s->rb());
+    }
     prof_mark(s, 2, stream);
     CHECK_LAUNCH();
     return 0;
@@ -816,6 +835,7 @@ int loop_close(pycfd_solver* s) {
 // A e = r in FP32 storage with the FP32 copy of the hierarchy to a relative
 // inner_tol and adds e to x.  Recorded, the outer loop and the inner CG loop
 // are nested WHILE nodes.
+
 constexpr int kIrMaxPasses = 40;
 constexpr int kInnerMaxIter = 200;
 
@@ -835,7 +855,7 @@ int solve_mixed(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
     pdl_launch(s, k_cg_pq<float, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r32, s->z32, s->pa32, s->pb32, s->q32, s->flags,
                                                           g, s->S, s->I, s->rb());
     CHECK_LAUNCH();
-    pdl_launch(s, k_cg_xr<float, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->x32, s->r32, s->pb32, s->q32, s->pa32, s->flags,
+    pdl_launch(s, k_cg_xr<float, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->x32, s->r32, s->pa32, s->pb32, s->q32, s->flags,
                                                           g, icfg, s->S, s->I, s->rb(), inner.ctl);
     CHECK_LAUNCH();
     return 0;
@@ -873,7 +893,9 @@ int solve_mixed(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
       if (!s->aux2) CU(cudaStreamCreateWithFlags(&s->aux2, cudaStreamNonBlocking));
       CU(cudaStreamBeginCaptureToGraph(s->aux2, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                        cudaStreamCaptureModeRelaxed));
+      const long long l0 = g_launches.load();
       TRY(inner_pass(s->aux2));
+      s->body_launches = g_launches.load() - l0;
       cudaGraph_t dummy = nullptr;
       CU(cudaStreamEndCapture(s->aux2, &dummy));
     }
@@ -983,11 +1005,12 @@ bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
     return false;
   for (int l = 1; l <= t; ++l)
     if (!d->levels[l].m_indptr) return false;
+  const bool mixed = s->precision == PCFD_MIXED;
   PatCycle<double> cd;
   PatCycle<float> cf;
   std::vector<std::function<bool()>> tasks;
   if (!pat_tasks<double>(d->levels, t, false, s->hflags.data(), &cd, &tasks)) return false;
-  if (s->precision == PCFD_MIXED && !pat_tasks<float>(d->levels, t, false, s->hflags.data(), &cf, &tasks)) return false;
+  if (mixed && !pat_tasks<float>(d->levels, t, false, s->hflags.data(), &cf, &tasks)) return false;
   if (!run_tasks(tasks)) return false;
   auto keep = [&](auto& c, auto& dn, auto& up) -> int {
     dn.resize(t + 1);
@@ -999,7 +1022,7 @@ bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
     return 0;
   };
   if ((*rc = keep(cd, s->pdn, s->pup))) return false;
-  if (s->precision == PCFD_MIXED && (*rc = keep(cf, s->pdnf, s->pupf))) return false;
+  if (mixed && (*rc = keep(cf, s->pdnf, s->pupf))) return false;
   return true;
 }
 
@@ -1057,14 +1080,27 @@ int cluster_shape(pycfd_solver* s) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0) {
+    // the answer depends on the device and the shape alone; asking takes milliseconds
+    static std::mutex mu;
+    static std::map<std::array<long, 4>, int> known;
+    std::lock_guard<std::mutex> hold(mu);
+    const std::array<long, 4> key{dev, C, cells, (long)smem};
+    auto it = known.find(key);
+    if (it == known.end()) {
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      if (known.size() >= 256) known.clear();
+      it = known.emplace(key, n).first;
+    }
+    if (it->second > 0) {
       s->cl_ctas = C;
       s->cl_cells = cells;
       s->cl_rmax = rmax;
       return 0;
     }
-    cudaGetLastError();
   }
   return 0;
 }
@@ -1108,22 +1144,22 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
     pdl_launch(s, k_rhs_init<double>, s->cgrid, s->cblock, 0, stream, s->b, x, s->r, s->flags, g, cfg, has_x0, s->S,
                                                       s->I, s->rb(), L.ctl);
     CHECK_LAUNCH();
-    // one pass of the recurrence on stream `st`; p_old -> p_new
-    auto pass = [&](cudaStream_t st, double* p_old, double* p_new, double* keep) -> int {
+    // one pass of the recurrence on stream `st`
+    auto pass = [&](cudaStream_t st) -> int {
       if (kind == PCFD_SOLVER_CG) {
-        pdl_launch(s, k_cg_pq<double, PC_JACOBI>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r, nullptr, p_old, p_new, s->q, s->flags,
+        pdl_launch(s, k_cg_pq<double, PC_JACOBI>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r, nullptr, s->pa, s->pb, s->q, s->flags,
                                                               g, s->S, s->I, s->rb());
         CHECK_LAUNCH();
-        pdl_launch(s, k_cg_xr<double, PC_JACOBI>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, x, s->r, p_new, s->q, keep, s->flags, g, cfg,
+        pdl_launch(s, k_cg_xr<double, PC_JACOBI>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, x, s->r, s->pa, s->pb, s->q, s->flags, g, cfg,
                                                               s->S, s->I, s->rb(), L.ctl);
       } else {
         TRY(vcycle_pcg<double>(s, s->r, s->z, st));
         prof_mark(s, 1, st);
-        pdl_launch(s, k_cg_pq<double, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r, s->z, p_old, p_new, s->q, s->flags, g,
+        pdl_launch(s, k_cg_pq<double, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r, s->z, s->pa, s->pb, s->q, s->flags, g,
                                                           s->S, s->I, s->rb());
         prof_mark(s, 1, st);
         CHECK_LAUNCH();
-        pdl_launch(s, k_cg_xr<double, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, x, s->r, p_new, s->q, keep, s->flags, g, cfg,
+        pdl_launch(s, k_cg_xr<double, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, x, s->r, s->pa, s->pb, s->q, s->flags, g, cfg,
                                                           s->S, s->I, s->rb(), L.ctl);
       }
       CHECK_LAUNCH();
@@ -1133,16 +1169,15 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
       TRY(launch_cg_cluster(s, x, stream));
     } else if (cap) {
       TRY(loop_open(s, stream, &L));
-      TRY(pass(s->aux, s->pa, s->pb, s->pa));
+      const long long l0 = g_launches.load();
+      TRY(pass(s->aux));
+      s->body_launches = g_launches.load() - l0;
       TRY(loop_close(s));
     } else {
-      double* pc = s->pa;
-      double* po = s->pb;
       for (;;) {
         TRY(read_flags(s, stream));
         if (s->hI[I_DONE]) break;
-        TRY(pass(stream, pc, po, nullptr));
-        std::swap(pc, po);
+        TRY(pass(stream));
       }
     }
     pdl_launch(s, k_finish_stats<double>, s->cgrid, s->cblock, 0, stream, x, s->b, s->flags, g, cfg, 1, s->S, s->I, s->rb());
@@ -1171,7 +1206,9 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
       };
       if (cap) {
         TRY(loop_open(s, stream, &L));
+        const long long l0 = g_launches.load();
         TRY(cycle(s->aux));
+        s->body_launches = g_launches.load() - l0;
         TRY(loop_close(s));
       } else {
         for (;;) {
@@ -1217,6 +1254,60 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
   return 0;
 }
 
+// The solve of a call that is not recorded whole.  Its iteration loop runs on the host --
+// one read of the done flag per pass -- for a solver's first solves, and as a recorded
+// solve with the loop on the device from then on, so that a solver used for a few solves
+// does not pay for the recording (about two steps' worth of solves; 128x128 MG-PCG step
+// 1.58 -> 1.20 ms).  Recorded solves are kept per iterate buffer (the solver's own) and
+// warm start.  Per-kernel timing needs the host loop.
+constexpr int kHostSolves = 6;
+int solve_rhs(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
+  auto direct = [&](cudaStream_t st) {
+    return s->precision == PCFD_MIXED ? solve_mixed(s, x, has_x0, st) : solve_prepared(s, x, has_x0, st);
+  };
+  if (s->capturing || s->prof_id || s->persistent || s->cl_ctas || s->solver_kind == PCFD_SOLVER_JACOBI ||
+      s->solver_kind == PCFD_SOLVER_SOR || s->host_solves < kHostSolves) {
+    if (!s->capturing) ++s->host_solves;
+    return direct(stream);
+  }
+  pycfd_solver::SolveGraph* hit = nullptr;
+  for (auto& e : s->solve_graphs)
+    if (e.x == x && e.has_x0 == has_x0) hit = &e;
+  if (!hit) {
+    if (!s->aux) CU(cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking));
+    if (!s->rec) CU(cudaStreamCreateWithFlags(&s->rec, cudaStreamNonBlocking));
+    pycfd_solver::SolveGraph e{};
+    e.x = x;
+    e.has_x0 = has_x0;
+    CU(cudaStreamBeginCapture(s->rec, cudaStreamCaptureModeThreadLocal));
+    s->capturing = true;
+    s->body_launches = 0;
+    const long long l0 = g_launches.load();
+    const int rc = direct(s->rec);
+    s->capturing = false;
+    const long long all = g_launches.load() - l0;
+    const cudaError_t ec = cudaStreamEndCapture(s->rec, &e.graph);
+    if (rc) {
+      if (e.graph) cudaGraphDestroy(e.graph);
+      return rc;
+    }
+    if (ec != cudaSuccess) return fail(PCFD_E_CUDA, "solve capture failed: %s", cudaGetErrorString(ec));
+    if (cudaGraphInstantiate(&e.exec, e.graph, 0) != cudaSuccess) {
+      cudaGraphDestroy(e.graph);
+      return fail(PCFD_E_CUDA, "solve recording failed: %s", cudaGetErrorString(cudaGetLastError()));
+    }
+    g_launches.fetch_sub(all);   // counted below, with every replay
+    e.body = s->body_launches;
+    e.fixed = all - e.body;
+    s->solve_graphs.push_back(e);
+    hit = &s->solve_graphs.back();
+  }
+  CU(cudaGraphLaunch(hit->exec, stream));
+  g_launches.fetch_add(hit->fixed);
+  s->replay_body = hit->body;    // times the iterations, once they are read (pycfd_get_stats)
+  return 0;
+}
+
 int set_dt(pycfd_solver* s, double dt, double blend, cudaStream_t stream) {
   // Step parameters live in device memory so a recorded step replays with new
   // values; they travel as kernel arguments, so no host synchronisation.
@@ -1232,8 +1323,7 @@ int project_impl(pycfd_solver* s, double* u, double* v, double* p, double dt_ove
   const int G = grid1(s);
   pdl_launch(s, k_div_rhs, s->cgrid, s->cblock, 0, stream, u, v, nullptr, s->flags, s->g, s->S, s->b, s->rb(), s->S);
   CHECK_LAUNCH();
-  if (s->precision == PCFD_MIXED) TRY(solve_mixed(s, s->x, s->has_guess, stream));
-  else TRY(solve_prepared(s, s->x, s->has_guess, stream));
+  TRY(solve_rhs(s, s->x, s->has_guess, stream));
   s->has_guess = true;
   const int gc = std::min(s->g.nx + 2, kMaxRedBlocks) + 1;   // rows + the ghost-ring block
   prof_mark(s, 7, stream);
@@ -1325,6 +1415,10 @@ int pycfd_solver_destroy(pycfd_solver* s) {
     cudaGraphExecDestroy(e.exec);
     cudaGraphDestroy(e.graph);
   }
+  for (auto& e : s->solve_graphs) {
+    cudaGraphExecDestroy(e.exec);
+    cudaGraphDestroy(e.graph);
+  }
   if (s->aux) cudaStreamDestroy(s->aux);
   if (s->rec) cudaStreamDestroy(s->rec);
   if (s->aux2) cudaStreamDestroy(s->aux2);
@@ -1410,7 +1504,8 @@ static int solver_create(const pycfd_solver_desc* d, bool member, pycfd_solver**
   {
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    s->pat_threads = (long)nsm * 2048;
+    s->pat_blocks = nsm * PCFD_PAT_MINB;
+    s->pat_threads = 256L * s->pat_blocks;
     // default: eight 256-thread blocks per SM (measured best of 4..12 on the 512^2 vortex;
     // with the ELL kernels' <= 48 registers five are resident, the rest follow as they end)
     s->ell_budget = d->ell_thread_budget ? (long)d->ell_thread_budget : (long)nsm * 8 * 256;
@@ -1703,7 +1798,7 @@ int pycfd_solver_momentum_rhs(pycfd_solver* s, const double* u, const double* v,
   if (s->les) return fail(PCFD_E_UNSUPPORTED, "use pycfd_momentum_rhs_les for the Smagorinsky closure");
   dim3 blk(TJ, TI), grd((g.ny + 1 + TJ - 1) / TJ, (g.nx + 1 + TI - 1) / TI);
   if (g.met) k_rhs_str<<<grd, blk, 0, st(stream)>>>(u, v, g, blend, rhs_u, rhs_v);
-  else k_rhs<<<grd, blk, 0, st(stream)>>>(u, v, g.nx, g.ny, g.dx, g.dy, g.nu, blend, g.fx, g.fy, rhs_u, rhs_v);
+  else k_rhs<<<grd, blk, 0, st(stream)>>>(u, v, g.nx, g.ny, RhsK(g.dx, g.dy, blend), g.nu, blend, g.fx, g.fy, rhs_u, rhs_v);
   CHECK_LAUNCH();
   return 0;
 }
@@ -1739,7 +1834,7 @@ int pycfd_momentum_rhs(const double* u, const double* v, int nx, int ny, double 
                        double blend, double fx, double fy, double* rhs_u, double* rhs_v, void* stream) {
   if (!u || !v || !rhs_u || !rhs_v || nx < 1 || ny < 1) return fail(PCFD_E_ARG, "bad arguments");
   dim3 blk(TJ, TI), grd((ny + 1 + TJ - 1) / TJ, (nx + 1 + TI - 1) / TI);
-  k_rhs<<<grd, blk, 0, st(stream)>>>(u, v, nx, ny, dx, dy, nu, blend, fx, fy, rhs_u, rhs_v);
+  k_rhs<<<grd, blk, 0, st(stream)>>>(u, v, nx, ny, RhsK(dx, dy, blend), nu, blend, fx, fy, rhs_u, rhs_v);
   CHECK_LAUNCH();
   return 0;
 }
@@ -1771,8 +1866,9 @@ int pycfd_momentum_rhs_les(const double* u, const double* v, int nx, int ny, dou
 int pycfd_divergence(const double* u, const double* v, int nx, int ny, double dx, double dy, double* out,
                      void* stream) {
   if (!u || !v || !out || nx < 1 || ny < 1) return fail(PCFD_E_ARG, "bad arguments");
-  dim3 cg, cb;
-  cell_launch(nx, ny, &cg, &cb);
+  // one cell per thread: its four loads are all there is to overlap (a wave of blocks
+  // striding over 16 cells each takes 18 us at 1500x1100 against 15)
+  const dim3 cb(kCellTJ, kCellTI), cg((ny + kCellTJ - 1) / kCellTJ, std::min(65535, (nx + kCellTI - 1) / kCellTI));
   k_divergence<<<cg, cb, 0, st(stream)>>>(u, v, nx, ny, dx, dy, out);
   CHECK_LAUNCH();
   return 0;
@@ -1794,8 +1890,7 @@ int pycfd_poisson_solve(pycfd_solver* s, const double* rhs, const double* p0, do
   pdl_launch(s, k_div_rhs, s->cgrid, s->cblock, 0, sm, nullptr, nullptr, rhs, s->flags, s->g, s->S, s->b, s->rb(), s->S);
   CHECK_LAUNCH();
   if (p0) CU(cudaMemcpyAsync(s->x_api, p0, s->ncell() * sizeof(double), cudaMemcpyDeviceToDevice, sm));
-  if (s->precision == PCFD_MIXED) TRY(solve_mixed(s, s->x_api, p0 != nullptr, sm));
-  else TRY(solve_prepared(s, s->x_api, p0 != nullptr, sm));
+  TRY(solve_rhs(s, s->x_api, p0 != nullptr, sm));
   CU(cudaMemcpyAsync(p, s->x_api, s->ncell() * sizeof(double), cudaMemcpyDeviceToDevice, sm));
   return 0;
 }
@@ -2298,6 +2393,8 @@ int pycfd_get_stats(pycfd_solver* s, pycfd_stats* o, void* stream) {
     o->body_fy[b] = s->hS[S_BODY_FY + b];
   }
   o->ir_iterations = s->hI[I_IR_IT];
+  if (s->replay_body) g_launches.fetch_add(s->replay_body * s->hI[I_TOTAL_IT]);   // replayed solves of this call
+  s->replay_body = 0;
   return 0;
 }
 

@@ -24,25 +24,34 @@ struct StageIn {
   }
 };
 
+// What a momentum right-hand side divides by or scales with: the spacings, their squares
+// and blend / dx, blend / dy (0 without the donor-cell part), formed once per thread or on
+// the host instead of at each of the two faces.
+struct RhsK {
+  double dx, dy, dx2, dy2, bx, by;
+  __host__ __device__ __forceinline__ RhsK(double x, double y, double blend)
+      : dx(x), dy(y), dx2(x * x), dy2(y * y), bx(blend > 0.0 ? blend / x : 0.0), by(blend > 0.0 ? blend / y : 0.0) {}
+};
+
 // u-momentum RHS at a u face from the values it reads (pycfd/core/kernels.py:54-80):
 // the face's own value, its east/west/north/south neighbours, and the four v faces
 // around it (v_tl = v[m-1, j+1], v_tr = v[m, j+1], v_bl = v[m-1, j], v_br = v[m, j]).
 __device__ __forceinline__ double rhs_u_core(double u0, double ue, double uw, double un, double us, double v_tl,
-                                             double v_tr, double v_bl, double v_br, double dx, double dy,
-                                             double nu, double blend, double fx) {
+                                             double v_tr, double v_bl, double v_br, const RhsK& k, double nu, double blend,
+                                             double fx) {
   const double u_right = 0.5 * (u0 + ue);
   const double u_left = 0.5 * (uw + u0);
-  double duudx = (rmul(u_right, u_right) - rmul(u_left, u_left)) / dx;
+  double duudx = (rmul(u_right, u_right) - rmul(u_left, u_left)) / k.dx;
   const double u_top = 0.5 * (u0 + un);
   const double v_top = 0.5 * (v_tl + v_tr);
   const double u_bot = 0.5 * (us + u0);
   const double v_bot = 0.5 * (v_bl + v_br);
-  double duvdy = (rmul(u_top, v_top) - rmul(u_bot, v_bot)) / dy;
+  double duvdy = (rmul(u_top, v_top) - rmul(u_bot, v_bot)) / k.dy;
   if (blend > 0.0) {
-    duudx += rmul(blend / dx, rmul(fabs(u_right), u0 - ue) * 0.5 - rmul(fabs(u_left), uw - u0) * 0.5);
-    duvdy += rmul(blend / dy, rmul(fabs(v_top), u0 - un) * 0.5 - rmul(fabs(v_bot), us - u0) * 0.5);
+    duudx += rmul(k.bx, rmul(fabs(u_right), u0 - ue) * 0.5 - rmul(fabs(u_left), uw - u0) * 0.5);
+    duvdy += rmul(k.by, rmul(fabs(v_top), u0 - un) * 0.5 - rmul(fabs(v_bot), us - u0) * 0.5);
   }
-  const double lap = ((uw - 2.0 * u0 + ue) / (dx * dx) + (us - 2.0 * u0 + un) / (dy * dy));
+  const double lap = ((uw - 2.0 * u0 + ue) / k.dx2 + (us - 2.0 * u0 + un) / k.dy2);
   return -(duudx + duvdy) + rmul(nu, lap) + fx;
 }
 
@@ -50,44 +59,42 @@ __device__ __forceinline__ double rhs_u_core(double u0, double ue, double uw, do
 // face, its north/south/east/west neighbours, and the four u faces around it
 // (u_rb = u[i+1, n-1], u_rt = u[i+1, n], u_lb = u[i, n-1], u_lt = u[i, n]).
 __device__ __forceinline__ double rhs_v_core(double v0, double vn, double vs, double ve, double vw, double u_rb,
-                                             double u_rt, double u_lb, double u_lt, double dx, double dy,
-                                             double nu, double blend, double fy) {
+                                             double u_rt, double u_lb, double u_lt, const RhsK& k, double nu, double blend,
+                                             double fy) {
   const double v_top = 0.5 * (v0 + vn);
   const double v_bot = 0.5 * (vs + v0);
-  double dvvdy = (rmul(v_top, v_top) - rmul(v_bot, v_bot)) / dy;
+  double dvvdy = (rmul(v_top, v_top) - rmul(v_bot, v_bot)) / k.dy;
   const double u_right = 0.5 * (u_rb + u_rt);
   const double v_right = 0.5 * (v0 + ve);
   const double u_left = 0.5 * (u_lb + u_lt);
   const double v_left = 0.5 * (vw + v0);
-  double duvdx = (rmul(u_right, v_right) - rmul(u_left, v_left)) / dx;
+  double duvdx = (rmul(u_right, v_right) - rmul(u_left, v_left)) / k.dx;
   if (blend > 0.0) {
-    dvvdy += rmul(blend / dy, rmul(fabs(v_top), v0 - vn) * 0.5 - rmul(fabs(v_bot), vs - v0) * 0.5);
-    duvdx += rmul(blend / dx, rmul(fabs(u_right), v0 - ve) * 0.5 - rmul(fabs(u_left), vw - v0) * 0.5);
+    dvvdy += rmul(k.by, rmul(fabs(v_top), v0 - vn) * 0.5 - rmul(fabs(v_bot), vs - v0) * 0.5);
+    duvdx += rmul(k.bx, rmul(fabs(u_right), v0 - ve) * 0.5 - rmul(fabs(u_left), vw - v0) * 0.5);
   }
-  const double lap = ((vw - 2.0 * v0 + ve) / (dx * dx) + (vs - 2.0 * v0 + vn) / (dy * dy));
+  const double lap = ((vw - 2.0 * v0 + ve) / k.dx2 + (vs - 2.0 * v0 + vn) / k.dy2);
   return -(duvdx + dvvdy) + rmul(nu, lap) + fy;
 }
 
 // u-momentum RHS at u-face (m, j), 1<=m<=nx+1, 1<=j<=ny.
 template <class U, class V>
 __device__ __forceinline__ double rhs_u_at(const U& u, const V& v, int m, int j, int ny,
-                                           double dx, double dy, double nu, double blend,
+                                           const RhsK& k, double nu, double blend,
                                            double fx) {
   const long W = ny + 2, WV = ny + 3;
   return rhs_u_core(u[m * W + j], u[(m + 1) * W + j], u[(m - 1) * W + j], u[m * W + j + 1], u[m * W + j - 1],
-                    v[(m - 1) * WV + j + 1], v[m * WV + j + 1], v[(m - 1) * WV + j], v[m * WV + j], dx, dy, nu,
-                    blend, fx);
+                    v[(m - 1) * WV + j + 1], v[m * WV + j + 1], v[(m - 1) * WV + j], v[m * WV + j], k, nu, blend, fx);
 }
 
 // v-momentum RHS at v-face (i, n), 1<=i<=nx, 1<=n<=ny+1.
 template <class U, class V>
 __device__ __forceinline__ double rhs_v_at(const U& u, const V& v, int i, int n, int ny,
-                                           double dx, double dy, double nu, double blend,
+                                           const RhsK& k, double nu, double blend,
                                            double fy) {
   const long W = ny + 2, WV = ny + 3;
   return rhs_v_core(v[i * WV + n], v[i * WV + n + 1], v[i * WV + n - 1], v[(i + 1) * WV + n], v[(i - 1) * WV + n],
-                    u[(i + 1) * W + n - 1], u[(i + 1) * W + n], u[i * W + n - 1], u[i * W + n], dx, dy, nu,
-                    blend, fy);
+                    u[(i + 1) * W + n - 1], u[(i + 1) * W + n], u[i * W + n - 1], u[i * W + n], k, nu, blend, fy);
 }
 
 // ---- stretched mesh (pycfd/core/solver.py:336-466, the array path) ------------
@@ -402,13 +409,13 @@ __global__ void k_predictor_les(StageIn u, StageIn v, double* __restrict__ us, d
 
 // Stateless RHS into (nx+1, ny) and (nx, ny+1) blocks.
 __global__ void k_rhs(const double* __restrict__ u, const double* __restrict__ v, int nx, int ny,
-                      double dx, double dy, double nu, double blend, double fx, double fy,
+                      RhsK k, double nu, double blend, double fx, double fy,
                       double* __restrict__ rhs_u, double* __restrict__ rhs_v) {
   pdl_begin();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;   // 0..ny
   const int i = blockIdx.y * blockDim.y + threadIdx.y;   // 0..nx
-  if (i <= nx && j < ny) rhs_u[(long)i * ny + j] = rhs_u_at(u, v, i + 1, j + 1, ny, dx, dy, nu, blend, fx);
-  if (i < nx && j <= ny) rhs_v[(long)i * (ny + 1) + j] = rhs_v_at(u, v, i + 1, j + 1, ny, dx, dy, nu, blend, fy);
+  if (i <= nx && j < ny) rhs_u[(long)i * ny + j] = rhs_u_at(u, v, i + 1, j + 1, ny, k, nu, blend, fx);
+  if (i < nx && j <= ny) rhs_v[(long)i * (ny + 1) + j] = rhs_v_at(u, v, i + 1, j + 1, ny, k, nu, blend, fy);
 }
 
 // Stateless RHS of a stretched mesh.
@@ -433,12 +440,13 @@ __global__ void k_predictor(StageIn u, StageIn v, double* __restrict__ us, doubl
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = g.nx, ny = g.ny;
   const double dt = S[S_DT], blend = S[S_BLEND];
+  const RhsK kc(g.dx, g.dy, blend);
   if (i < nx + 3 && j < ny + 2) {
     const long k = (long)i * (ny + 2) + j;
     double val = u[k];
     if (i >= g.u_lo && i < g.u_hi && j >= 1 && j <= ny)
       val = val + rmul(dt, g.met ? rhs_u_str(u, v, i, j, ny, Metrics(g), g.nu, blend, g.fx)
-                                 : rhs_u_at(u, v, i, j, ny, g.dx, g.dy, g.nu, blend, g.fx));
+                                 : rhs_u_at(u, v, i, j, ny, kc, g.nu, blend, g.fx));
     us[k] = val;
   }
   if (i < nx + 2 && j < ny + 3) {
@@ -446,7 +454,7 @@ __global__ void k_predictor(StageIn u, StageIn v, double* __restrict__ us, doubl
     double val = v[k];
     if (i >= 1 && i <= nx && j >= g.v_lo && j < g.v_hi)
       val = val + rmul(dt, g.met ? rhs_v_str(u, v, i, j, ny, Metrics(g), g.nu, blend, g.fy)
-                                 : rhs_v_at(u, v, i, j, ny, g.dx, g.dy, g.nu, blend, g.fy));
+                                 : rhs_v_at(u, v, i, j, ny, kc, g.nu, blend, g.fy));
     vs[k] = val;
   }
 }

@@ -77,10 +77,16 @@ class GpuOptions:
     ell_thread_budget: int = 0
 
 
+_found = []   # torch, once it has a CUDA device (asking it again costs a driver call per method)
+
+
 def _torch():
+    if _found:
+        return _found[0]
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("pycfd_b200 needs a CUDA device; there is no CPU fallback")
+    _found.append(torch)
     return torch
 
 
@@ -492,6 +498,8 @@ class ProjectionSolver:
     def _dev(self, a):
         torch = _torch()
         if isinstance(a, torch.Tensor):
+            if a.dtype is torch.float64 and a.device.type == "cuda" and a.device.index == torch.cuda.current_device():
+                return a
             return a.to(device="cuda", dtype=torch.float64)
         return torch.as_tensor(np.asarray(a, dtype=np.float64), device="cuda")
 
