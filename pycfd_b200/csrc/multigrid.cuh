@@ -379,13 +379,13 @@ __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
   }
 }
 
-// Level 0: z = Q_0 x_1 + G_0 b_0 (b_0 the projected CG residual) with sum z and r.z for
-// the projected z and rho; a block walks `rounds` tiles along x.
+// Level 0: z = Q_0 x_1 + G_0 b_0 (b_0 the projected CG residual) with the partials of sum z
+// and r.z for the projected z and rho; a block walks `rounds` tiles along x.
 template <class T, bool F65>
 __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
     k_pat_up0(Pat<T> E, int rounds, const T* __restrict__ x1, const T* __restrict__ r,
-              const uint8_t* __restrict__ flags, Geo g, int singular, double* __restrict__ S, T* __restrict__ z,
-              RedBuf rb) {
+              const uint8_t* __restrict__ flags, int singular, const double* __restrict__ S, T* __restrict__ z,
+              double* __restrict__ zpart) {
   const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
   const int j = (int)blockIdx.x * 32 + lane, nx = E.n / E.ny_r;
   const int i1 = min(nx, ((int)blockIdx.y + 1) * rounds * 8);
@@ -424,12 +424,20 @@ __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
     }
     i += 8;
   }
-  grid_reduce<2>(acc, rb, [&](double* t) {
+  block_partial<2>(acc, zpart);
+}
+
+// Closes the sums of k_pat_up0 where no k_cg_pq follows (one cycle applied by itself).
+__global__ void k_up0_close(const double* __restrict__ zpart, int nz, Geo g, int singular, double* __restrict__ S) {
+  pdl_begin();
+  double t[2];
+  block_total<2>(zpart, nz, t);
+  if (threadIdx.x == 0) {
     const double m = (singular && g.n_fluid) ? t[0] / g.n_fluid : 0.0;
     S[S_MEAN_Z] = m;
     S[S_RHO_PREV] = S[S_RHO];
     S[S_RHO] = t[1] - m * S[S_SUM_R];
-  });
+  }
 }
 
 // x = wd*b and res = b - A(wd*b) on level 0.

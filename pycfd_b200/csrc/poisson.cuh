@@ -85,21 +85,37 @@ __global__ void k_rhs_init(double* __restrict__ b, T* __restrict__ x, T* __restr
   });
 }
 
+// nz > 0: the cycle's sums (sum z, r.z) are nz rows of partials at zpart, added here by
+// every block; p.q goes out as partials to k_cg_xr.  rho of pass `it` is left in slot
+// S_RHO2 + (it & 1).
 // p = z + beta p_old with z = r/d (Jacobi) or z = z_raw - mean_z on solvable
 // rows (multigrid; z_raw from the V-cycle), q = A p, and p.q -> alpha.
 // The direction of pass `it` is pa (it even) or pb (it odd), the previous one the other, so
 // no pass copies p and a recorded loop body reads the right one.
 template <class T, int PC>
 __global__ void k_cg_pq(const T* __restrict__ r, const T* __restrict__ zraw, T* pa, T* pb, T* __restrict__ q,
-                        const uint8_t* __restrict__ flags, Geo g, double* __restrict__ S,
-                        const int* __restrict__ I, RedBuf rb) {
+                        const uint8_t* __restrict__ flags, Geo g, int singular, double* __restrict__ S,
+                        const int* __restrict__ I, const double* __restrict__ zpart, int nz,
+                        double* __restrict__ qpart) {
   pdl_begin();
   const int it = I[I_IT];
   const bool first = it == 0;
   const T* __restrict__ p_old = (it & 1) ? pa : pb;
   T* __restrict__ p_new = (it & 1) ? pb : pa;
-  const double beta = first ? 0.0 : S[S_RHO] / S[S_RHO_PREV];
-  const double mz = S[S_MEAN_Z];
+  double beta, mz;
+  if (nz) {   // the cycle left its sums as partials
+    double t[2];
+    const double rho_prev = S[S_RHO2 + ((it + 1) & 1)], sum_r = S[S_SUM_R];
+    block_total<2>(zpart, nz, t);
+    mz = (singular && g.n_fluid) ? t[0] / g.n_fluid : 0.0;
+    const double rho = t[1] - mz * sum_r;
+    beta = first ? 0.0 : rho / rho_prev;
+    if (blockIdx.x == 0 && threadIdx.x == 0) S[S_RHO2 + (it & 1)] = rho;   // the other slot is being read
+  } else {
+    beta = first ? 0.0 : S[S_RHO] / S[S_RHO_PREV];
+    mz = S[S_MEAN_Z];
+    if (blockIdx.x == 0 && threadIdx.x == 0) S[S_RHO2 + (it & 1)] = S[S_RHO];
+  }
   auto pval = [&](int k, int ii, int jj) -> double {
     const uint8_t fk = flags[k];
     double z;
@@ -117,10 +133,7 @@ __global__ void k_cg_pq(const T* __restrict__ r, const T* __restrict__ zraw, T* 
                       q[c] = (T)qc;
                       acc[0] += pc * qc;
                     });
-  grid_reduce<1>(acc, rb, [&](double* t) {
-    S[S_PQ] = t[0];
-    S[S_ALPHA] = S[S_RHO] / t[0];
-  });
+  block_partial<1>(acc, qpart);
 }
 
 // x += alpha p, r -= alpha q; ||r||^2, r.(r/d), sum_solvable(r); convergence
@@ -128,10 +141,15 @@ __global__ void k_cg_pq(const T* __restrict__ r, const T* __restrict__ zraw, T* 
 template <class T, int PC>
 __global__ void k_cg_xr(T* __restrict__ x, T* __restrict__ r, const T* pa, const T* pb, const T* __restrict__ q,
                         const uint8_t* __restrict__ flags, Geo g, SolveCfg cfg,
-                        double* __restrict__ S, int* __restrict__ I, RedBuf rb, LoopCtl loop) {
+                        double* __restrict__ S, int* __restrict__ I, const double* __restrict__ qpart, int nq,
+                        RedBuf rb, LoopCtl loop) {
   pdl_begin();
-  const T* __restrict__ p = (I[I_IT] & 1) ? pb : pa;
-  const double alpha = S[S_ALPHA];
+  const int it0 = I[I_IT];
+  const T* __restrict__ p = (it0 & 1) ? pb : pa;
+  const double rho = S[S_RHO2 + (it0 & 1)];
+  double pq[1];
+  block_total<1>(qpart, nq, pq);
+  const double alpha = rho / pq[0];
   double acc[3] = {0, 0, 0};
   T pv[kStripRows], xv[kStripRows], rv[kStripRows], qv[kStripRows];
   uint8_t fv[kStripRows];

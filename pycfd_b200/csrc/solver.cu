@@ -217,6 +217,9 @@ struct pycfd_solver {
 
   dim3 cgrid, cblock;   // 2D launch over the fine cells
   RedBuf rb() const { return RedBuf{partials, counter}; }
+  double* qpart() const { return partials + (size_t)kPartPq * kMaxRedBlocks; }
+  double* zpart = nullptr;   // partials of the level-0 up product
+  int nz = 0;   // rows of partials the last recorded or launched cycle leaves (0: sums closed)
   SolveCfg cfg() const { return SolveCfg{tol, maxiter, singular, 0}; }
   long ncell() const { return (long)g.nx * g.ny; }
 };
@@ -506,6 +509,7 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
     CHECK_LAUNCH();
     return 0;
   }
+  s->nz = 0;
   if (!patDn<T>(s).empty()) {
     const int tl = s->tail_level;
     auto product = [&](const Pat<T>& E, const T* s1, const T* s2, T* y, bool from_r) -> int {
@@ -531,7 +535,8 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
       const int rounds = (int)((tiles + s->pat_blocks - 1) / s->pat_blocks);   // one wave of blocks
       const dim3 grid(q.grid.x, (q.grid.y + rounds - 1) / rounds);
       pdl_launch(s, pat_is_65(E) ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds,
-                 (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, g, s->singular, s->S, z_out, s->rb());
+                 (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, s->singular, (const double*)s->S, z_out, s->zpart);
+      s->nz = (int)(grid.x * grid.y);
     }
     prof_mark(s, 2, stream);
     CHECK_LAUNCH();
@@ -853,10 +858,10 @@ int solve_mixed(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
   auto inner_pass = [&](cudaStream_t st) -> int {
     TRY(vcycle_pcg<float>(s, s->r32, s->z32, st));
     pdl_launch(s, k_cg_pq<float, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r32, s->z32, s->pa32, s->pb32, s->q32, s->flags,
-                                                          g, s->S, s->I, s->rb());
+                                                          g, s->singular, s->S, s->I, (const double*)s->zpart, s->nz, s->qpart());
     CHECK_LAUNCH();
     pdl_launch(s, k_cg_xr<float, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->x32, s->r32, s->pa32, s->pb32, s->q32, s->flags,
-                                                          g, icfg, s->S, s->I, s->rb(), inner.ctl);
+                                                          g, icfg, s->S, s->I, (const double*)s->qpart(), strip_grid(s->g), s->rb(), inner.ctl);
     CHECK_LAUNCH();
     return 0;
   };
@@ -995,7 +1000,8 @@ int solve_persistent(pycfd_solver* s, double* x, bool has_x0, cudaStream_t strea
 
 // The V-cycle of an MG-PCG solver as pattern products, where its form allows: one sweep
 // per level, a dense tail, fused restrictions asked for, no other form of the coarse
-// levels, a uniform mesh (on a stretched one every row differs) and few enough patterns.
+// levels, a uniform mesh (on a stretched one every row differs: 301x147 steps in 1.88 ms
+// with a pattern per row, 1.75 with the stored operators) and few enough patterns.
 // They then take the place of the level operators, which are not uploaded.
 bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
   *rc = 0;
@@ -1021,6 +1027,8 @@ bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
     }
     return 0;
   };
+  // (sum z, r.z) per block of the level-0 product: one wave of blocks, rounded up per column of tiles
+  if ((*rc = dalloc(s, &s->zpart, 2 * ((size_t)s->pat_blocks + (s->g.ny + 31) / 32 + 1)))) return false;
   if ((*rc = keep(cd, s->pdn, s->pup))) return false;
   if (mixed && (*rc = keep(cf, s->pdnf, s->pupf))) return false;
   return true;
@@ -1148,19 +1156,19 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
     auto pass = [&](cudaStream_t st) -> int {
       if (kind == PCFD_SOLVER_CG) {
         pdl_launch(s, k_cg_pq<double, PC_JACOBI>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r, nullptr, s->pa, s->pb, s->q, s->flags,
-                                                              g, s->S, s->I, s->rb());
+                                                              g, s->singular, s->S, s->I, (const double*)nullptr, 0, s->qpart());
         CHECK_LAUNCH();
         pdl_launch(s, k_cg_xr<double, PC_JACOBI>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, x, s->r, s->pa, s->pb, s->q, s->flags, g, cfg,
-                                                              s->S, s->I, s->rb(), L.ctl);
+                                                              s->S, s->I, (const double*)s->qpart(), strip_grid(s->g), s->rb(), L.ctl);
       } else {
         TRY(vcycle_pcg<double>(s, s->r, s->z, st));
         prof_mark(s, 1, st);
         pdl_launch(s, k_cg_pq<double, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, s->r, s->z, s->pa, s->pb, s->q, s->flags, g,
-                                                          s->S, s->I, s->rb());
+                                                          s->singular, s->S, s->I, (const double*)s->zpart, s->nz, s->qpart());
         prof_mark(s, 1, st);
         CHECK_LAUNCH();
         pdl_launch(s, k_cg_xr<double, PC_MG>, dim3(strip_grid(s->g)), dim3(kStripThreads), 0, st, x, s->r, s->pa, s->pb, s->q, s->flags, g, cfg,
-                                                          s->S, s->I, s->rb(), L.ctl);
+                                                          s->S, s->I, (const double*)s->qpart(), strip_grid(s->g), s->rb(), L.ctl);
       }
       CHECK_LAUNCH();
       return 0;
@@ -1908,6 +1916,10 @@ int pycfd_mg_apply(pycfd_solver* s, const double* r, double* z, void* stream) {
   CU(cudaMemsetAsync(s->S + S_SUM_R, 0, sizeof(double), sm));
   CU(cudaMemsetAsync(s->I + I_ZERO_RHS, 0, sizeof(int), sm));
   TRY(vcycle_pcg<double>(s, r, s->z, sm));
+  if (s->nz) {
+    pdl_launch(s, k_up0_close, 1, 256, 0, sm, (const double*)s->zpart, s->nz, s->g, s->singular, s->S);
+    CHECK_LAUNCH();
+  }
   // z = z_raw - mean_z on solvable rows, 0 elsewhere
   CU(cudaMemcpyAsync(s->S + S_MEAN_X, s->S + S_MEAN_Z, sizeof(double), cudaMemcpyDeviceToDevice, sm));
   pdl_launch(s, k_finish_apply<double>, s->cgrid, s->cblock, 0, sm, s->z, z, s->flags, s->g, s->S, s->I);
