@@ -259,7 +259,9 @@ class BatchOptions:
     coarse_level: int = 0        #: multigrid levels from this one down: one block per problem (0: off)
     coarse_tail: bool = True     #: close each structure's V-cycle with its dense tail operator
     tail_ratio: float | None = 16.0   #: bound the tail operator: n_t^2 <= tail_ratio * n_0 (None: none)
-    fused_restriction: bool = False   #: down sweep by R (I - A W) products (one sweep, every structure tailed)
+    #: down sweep by R (I - A W) products (one sweep, every structure tailed); the row-pattern
+    #: form (one sweep, fused_from 1, ell_group 8, no coarse_level or stencil transfer) always does
+    fused_restriction: bool = False
     fused_from: int = 1               #: first level so restricted (2: the fine level's restriction stays)
     ell_group: int = 8                #: problems per coarse-level block sharing the matrix loads (1 or 8)
     programmatic_launch: bool = False  #: programmatic dependent launch between the kernels (off: plain order)

@@ -20,7 +20,8 @@
 // launch per level and direction and stores one vector per level and direction.
 // Measured on B200 against the stored operators (ms per step): 512x512 vortex 2.67 ->
 // 1.91, 2048x1024 cylinder 15.9 -> 10.2, 512x256 cylinder in the mixed form 2.39 -> 2.06;
-// batches: 64 cavities in FP64 7.48 -> 4.16, 256 mixed 13.0 -> 10.4, 24 odd 5.4 -> 3.5.
+// batches: 64 cavities in FP64 7.48 -> 4.16, 256 mixed 13.0 -> 10.4, 24 odd 5.4 -> 3.5
+// (with entries in units of four, tiles and groups 2.8).
 #pragma once
 #include "common.cuh"
 
