@@ -320,7 +320,20 @@ def batch_cpu_baseline(cfgs, steps=1, warmup=0, workers=None):
                       f"{warmup} untimed step(s), timed together ({wall:.1f} s wall)"}
 
 
-def batch_kernel_bytes(kid, cells, its, s_bytes):
+def row_patterns(opts):
+    """Whether a batch of these options runs its V-cycle as row-pattern products, whose
+    level-0 up product is the kernel of kind 2."""
+    return (opts.mg_sweeps == 1 and opts.ell_group == 8 and opts.fused_from == 1
+            and opts.coarse_level == 0 and not opts.stencil_transfer)
+
+
+def kernel_name(kid, patterns):
+    if kid == 2 and patterns:
+        return "k_b_up0 (level-0 up product z = Q x1 + G r, and r.z)"
+    return KERNEL_NAMES[kid]
+
+
+def batch_kernel_bytes(kid, cells, its, s_bytes, patterns=False):
     """Algorithmic bytes of one eager step's launches of kernel kind `kid` (ids of
     pycfd_batch_profile), from each problem's CG passes in that step."""
     passes = float((its * cells).sum())
@@ -328,6 +341,8 @@ def batch_kernel_bytes(kid, cells, its, s_bytes):
         return passes * (4 * s_bytes + 1)
     if kid == 5:     # k_b_cg_xr: read p, x, r, q, flags; write x, r
         return passes * (6 * s_bytes + 1)
+    if kid == 2 and patterns:   # k_b_up0: read x1 (a quarter of the cells), r, flags; write z
+        return passes * (2.25 * s_bytes + 1)
     if kid == 2:     # k_b_fine (last sweep): read x0, r, flags; write z
         return passes * (3 * s_bytes + 1)
     if kid == 3:     # k_b_fine (first sweep): read r, flags; write x0, lres0
@@ -416,11 +431,11 @@ def run_batch(args, world, rank, local):
     # roofline: the kernel kind with the largest share of one eager step
     s_bytes = 4 if opts.precision == "mixed" else 8
     cells = np.array([c.nx * c.ny for c in cfgs], dtype=np.float64)
-    prof = {}
+    prof, pats = {}, row_patterns(opts)
     if not args.no_profile:
         for kid in (1, 2, 3, 5, 6):
             kms, kn, kits = b.profile(kid, 1)
-            prof[kid] = (kms, kn, batch_kernel_bytes(kid, cells, kits, s_bytes))
+            prof[kid] = (kms, kn, batch_kernel_bytes(kid, cells, kits, s_bytes, pats))
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -438,16 +453,16 @@ def run_batch(args, world, rank, local):
         traffic = None
         try:
             tr = json.load(open(os.path.join(ROOT, "profiles", "roofline_traffic.json")))
-            traffic = tr.get("batch_" + opts.precision, {}).get(str(top))
+            traffic = tr.get("batch_" + opts.precision, {}).get("2p" if top == 2 and pats else str(top))
         except Exception:
             pass
-        roof = {"bound": "hbm", "kernel": KERNEL_NAMES[top], "achieved": achieved, "peak": hbm,
+        roof = {"bound": "hbm", "kernel": kernel_name(top, pats), "achieved": achieved, "peak": hbm,
                 "unit": "GB/s", "frac": achieved / hbm if achieved else None, "traffic": traffic,
                 "bytes_per_launch": kbytes / max(kn, 1), "us_per_launch": 1e3 * kms / max(kn, 1),
                 "launches": kn, "peak_source": peak_src,
                 "timing": "CUDA events around each eager launch of the kernel over one step; bytes = "
                           "sum over problems of its passes x cells x bytes per cell",
-                "kernels": {KERNEL_NAMES[k].split(" ")[0] + ("" if k not in (2, 3) else f"[{k}]"):
+                "kernels": {kernel_name(k, pats).split(" ")[0] + ("" if k not in (2, 3) else f"[{k}]"):
                             {"ms": v[0], "launches": v[1],
                              "gb_s": (v[2] / (v[0] / 1e3) / 1e9) if v[0] > 0 and v[2] else None}
                             for k, v in prof.items()},
@@ -460,9 +475,9 @@ def run_batch(args, world, rank, local):
             one = {}
             for kid in prof:
                 kms1, kn1, kits1 = b1.profile(kid, 1)
-                kb1 = batch_kernel_bytes(kid, cells, kits1, s_bytes)
+                kb1 = batch_kernel_bytes(kid, cells, kits1, s_bytes, pats)
                 gbs = kb1 / (kms1 / 1e3) / 1e9 if kms1 > 0 and kb1 else None
-                one[KERNEL_NAMES[kid].split(" ")[0] + ("" if kid not in (2, 3) else f"[{kid}]")] = {
+                one[kernel_name(kid, pats).split(" ")[0] + ("" if kid not in (2, 3) else f"[{kid}]")] = {
                     "us_per_launch": 1e3 * kms1 / max(kn1, 1), "launches": kn1, "gb_s": gbs,
                     "frac": gbs / hbm if gbs else None}
             del b1
