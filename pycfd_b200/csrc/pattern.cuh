@@ -31,15 +31,27 @@ template <class T> struct PatEntry;
 template <> struct alignas(8) PatEntry<float> { int off; float val; };
 template <> struct alignas(16) PatEntry<double> { double val; int off; int pad; };
 
-__device__ __forceinline__ void pat_load(const PatEntry<float>* e, int* off, float* val) {
+// The walks over a row's entries below compile for the host too, where the tables are
+// checked against the products they hold.
+__host__ __device__ __forceinline__ void pat_load(const PatEntry<float>* e, int* off, float* val) {
+#ifdef __CUDA_ARCH__
   const int2 w = __ldg(reinterpret_cast<const int2*>(e));
   *off = w.x;
   *val = __int_as_float(w.y);
+#else
+  *off = e->off;
+  *val = e->val;
+#endif
 }
-__device__ __forceinline__ void pat_load(const PatEntry<double>* e, int* off, double* val) {
+__host__ __device__ __forceinline__ void pat_load(const PatEntry<double>* e, int* off, double* val) {
+#ifdef __CUDA_ARCH__
   const int4 w = __ldg(reinterpret_cast<const int4*>(e));
   *val = __hiloint2double(w.y, w.x);
   *off = w.z;
+#else
+  *off = e->off;
+  *val = e->val;
+#endif
 }
 
 // How a row's base index follows from the row: its own index, the cell of the coarser
@@ -49,7 +61,9 @@ enum PatBase { PB_SAME = 0, PB_COARSER = 1, PB_FINER = 2 };
 // An operator of one source (K2 = 0), or of two: K entries on the first from its base
 // index, then K2 on the second, a vector on the rows' own grid.  Both counts are padded to
 // units of four entries (kPatUnit), so that no entry needs a test of its own -- except the
-// level-0 up product of 2 x 2 aggregates, whose 6 + 5 entries have code of their own.
+// level-0 up product of 2 x 2 aggregates, whose 6 + 5 entries have code of their own in the
+// level-0 kernels (f65).  A coarse level can have rows of 6 and 5 entries too (level 1 of
+// a one-cell channel with a bend): its tables are in units, as its kernels read them.
 template <class T>
 struct Pat {
   const uint16_t* pid;        // pattern of each row
@@ -58,6 +72,7 @@ struct Pat {
   int base, ny_r, ny_c;       // PatBase; columns (y cells) of the row and the source grid
   int fx, fy;                 // coarsening factors between them (1 or 2)
   unsigned inv;               // ceil(2^32 / ny_r): rows are divided by a multiplication
+  int f65;                    // 1: 6 + 5 entries without padding (level-0 up product only)
 };
 constexpr int kPatUnit = 4;
 
@@ -86,8 +101,9 @@ __device__ __forceinline__ const PatEntry<T>* pat_tab(const Pat<T>& E, int row) 
 }
 
 // acc[g] += N entries of tb applied to x(g, index), all gathers issued before the sums.
+#pragma nv_exec_check_disable
 template <int N, int GS, class T, class A, class X>
-__device__ __forceinline__ void pat_batch(const PatEntry<T>* tb, int base, X x, A (&acc)[GS]) {
+__host__ __device__ __forceinline__ void pat_batch(const PatEntry<T>* tb, int base, X x, A (&acc)[GS]) {
   int at[N];
   T val[N];
   A xv[N][GS];
@@ -105,10 +121,11 @@ __device__ __forceinline__ void pat_batch(const PatEntry<T>* tb, int base, X x, 
 
 // Units [q0, q1) of a row (its table at tb): xa(g, index) gathers the first source, xb the
 // second, for GS members.  Up to 16 gathers are in flight together.
+#pragma nv_exec_check_disable
 template <int GS, class T, class A, class XA, class XB>
-__device__ __forceinline__ void pat_units(const Pat<T>& E, const PatEntry<T>* tb, int base, int row, int q0, int q1,
+__host__ __device__ __forceinline__ void pat_units(const Pat<T>& E, const PatEntry<T>* tb, int base, int row, int q0, int q1,
                                           XA xa, XB xb, A (&acc)[GS]) {
-  const int qa = min(q1, E.K / kPatUnit);
+  const int ka = E.K / kPatUnit, qa = q1 < ka ? q1 : ka;
   int q = q0;
   if constexpr (GS <= 2) {
     for (; q + 2 <= qa; q += 2) pat_batch<2 * kPatUnit, GS>(tb + q * kPatUnit, base, xa, acc);
@@ -132,10 +149,9 @@ __device__ __forceinline__ void pat_units(const Pat<T>& E, const PatEntry<T>* tb
 
 // The whole row: the level-0 up product of 2 x 2 aggregates (6 + 5 entries) by code of its
 // own, any other by units.
-template <class T>
-__host__ __device__ __forceinline__ bool pat_is_65(const Pat<T>& E) { return E.K == 6 && E.K2 == 5; }
+#pragma nv_exec_check_disable
 template <bool F65, int GS, class T, class A, class XA, class XB>
-__device__ __forceinline__ void pat_whole(const Pat<T>& E, const PatEntry<T>* tb, int row, XA xa, XB xb, A (&acc)[GS]) {
+__host__ __device__ __forceinline__ void pat_whole(const Pat<T>& E, const PatEntry<T>* tb, int row, XA xa, XB xb, A (&acc)[GS]) {
   const int base = pat_base(E, row);
   if constexpr (F65) {
     pat_batch<6, GS>(tb, base, xa, acc);

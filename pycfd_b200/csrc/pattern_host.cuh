@@ -221,8 +221,10 @@ struct PatHost {
 // rows, where a row with a pattern of its own would be read uncoalesced; smaller levels
 // stay in L1 and L2 whatever their patterns.  any: no such limit (a batch's groups read
 // an entry once for eight problems, and its problems must not change routes with size).
+// up0: the level-0 up product, whose kernels read 6 + 5 entries without padding.
 template <class T>
-bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t* liveB, bool any, PatHost<T>* out) {
+bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t* liveB, bool up0, bool any,
+               PatHost<T>* out) {
   Pat<T>& E = out->v;
   const int n = A.n;
   int K = 1, K2 = 0;
@@ -230,7 +232,8 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
     K = std::max<int>(K, (int)(A.ptr[r + 1] - A.ptr[r]));
     if (B) K2 = std::max<int>(K2, (int)(B->ptr[r + 1] - B->ptr[r]));
   }
-  if (!(K == 6 && K2 == 5)) {   // units of four entries (pattern.cuh)
+  E.f65 = up0 && K == 6 && K2 == 5;
+  if (!E.f65) {   // units of four entries (pattern.cuh)
     K = (K + kPatUnit - 1) / kPatUnit * kPatUnit;
     K2 = (K2 + kPatUnit - 1) / kPatUnit * kPatUnit;
   }
@@ -322,9 +325,9 @@ bool pat_tasks(const pycfd_mg_level* lv, int t, bool any, const uint8_t* flags, 
       Csr Q, G;
       up_products(*f, *c, &Q, &G);
       const CsrV g = G;
-      return pat_build<T>(Q, nullptr, &g, live, any, q);
+      return pat_build<T>(Q, nullptr, &g, live, l == 0, any, q);
     });
-    tasks->push_back([=]() { return pat_build<T>(down_product(*f, *c), live, nullptr, nullptr, any, m); });
+    tasks->push_back([=]() { return pat_build<T>(down_product(*f, *c), live, nullptr, nullptr, false, any, m); });
   }
   return true;
 }

@@ -534,7 +534,7 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
       const long tiles = (long)q.grid.x * q.grid.y;
       const int rounds = (int)((tiles + s->pat_blocks - 1) / s->pat_blocks);   // one wave of blocks
       const dim3 grid(q.grid.x, (q.grid.y + rounds - 1) / rounds);
-      pdl_launch(s, pat_is_65(E) ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds,
+      pdl_launch(s, E.f65 ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds,
                  (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, s->singular, (const double*)s->S, z_out, s->zpart);
       s->nz = (int)(grid.x * grid.y);
     }

@@ -1,0 +1,120 @@
+"""Tables of row patterns against the products they hold (no GPU needed).
+
+The library's own host code builds the tables of a hierarchy and walks them entry by
+entry as the kernels do; the walk must give M b, and Q x + G b, of every level in both
+storage types.  Bent channels are the masks where a coarse level's rows take the widths
+(6 and 5 entries) of the usual level-0 product.
+"""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import cases
+import native_build
+from pycfd_b200.config import BCKind, BCSpec, PressureSolver, SimulationConfig
+from pycfd_b200.hierarchy import hierarchy_for, tail_level
+from pycfd_b200.mesh import StructuredMesh
+from pycfd_b200.solver import BoundaryInfo, GpuOptions, native_desc
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    L = native_build.load("pattern_tables", tmp_path_factory.mktemp("native"))
+    L.pt_build.restype = C.c_void_p
+    L.pt_build.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_void_p]
+    L.pt_free.argtypes = [C.c_void_p]
+    L.pt_ok.argtypes = [C.c_void_p, C.c_int]
+    L.pt_info.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int)]
+    L.pt_apply.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    return L
+
+
+def channel(nx, ny, w, i, j):
+    """All solid but an L-shaped channel of width w with its corner at (i, j)."""
+    solid = np.ones((nx, ny), bool)
+    solid[i:i + w, j:] = False
+    solid[i:, j:j + w] = False
+    return solid
+
+
+def circle(nx, ny):
+    x, y = np.meshgrid(np.arange(nx) + 0.5, np.arange(ny) + 0.5, indexing="ij")
+    return (x - 0.4 * nx) ** 2 + (y - 0.5 * ny) ** 2 < (0.2 * min(nx, ny)) ** 2
+
+
+def problem(nx, ny, solid, ratio, bc=None):
+    """(levels, closing level, descriptor, what it points to, solvable cells)."""
+    cfg = cases.to_config(dict(nx=nx, ny=ny, lx=nx / 64.0, ly=ny / 64.0, re=100.0, pressure_solver="mgcg",
+                               boundary_config=bc or cases.bcs()), SimulationConfig, BCSpec, BCKind)
+    mesh = StructuredMesh.from_config(cfg)
+    bnd = BoundaryInfo(cfg.boundary_config, mesh)
+    op, (levels, cinv) = hierarchy_for(nx, ny, mesh.dx, mesh.dy, bnd.periodic_x, bnd.periodic_y, solid,
+                                       bnd.dirichlet_pressure() or None)
+    body = np.zeros((nx, ny), bool) if solid is None else solid
+    d, keep = native_desc(cfg, mesh, bnd, body, solid is not None, (), PressureSolver.MGCG,
+                          GpuOptions(tail_ratio=ratio), levels, cinv)
+    t = tail_level(levels, ratio) or len(levels) - 1
+    return levels, t, d, keep, np.asarray(op.fluid, np.uint8).ravel()
+
+
+def products(levels, l):
+    """M of level l + 1 and (Q, G) of level l, in double."""
+    f, P = levels[l], levels[l + 1].P.tocsr()
+    A, W = f.A.tocsr(), sp.diags(np.asarray(f.weighted_dinv))
+    eye = sp.identity(f.n, format="csr")
+    return P.T @ (eye - A @ W), (eye - W @ A) @ P, W @ (2.0 * eye - A @ W)
+
+
+CHANNELS = [(135, 145, 1, 3, 6, None), (151, 177, 1, 111, 110, None), (51, 71, 1, 14, 23, 16.0),
+            (13, 78, 1, 10, 0, 16.0)]
+
+
+def check(L, nx, ny, solid, ratio, bc=None):
+    levels, t, d, keep, solvable = problem(nx, ny, solid, ratio, bc)
+    rng = np.random.default_rng(nx * 1000 + ny)
+    h = L.pt_build(C.cast(d.levels, C.c_void_p), t, 1, solvable.ctypes.data)
+    raw = set()   # (level, widest row of Q, of G) as the products have them
+    try:
+        for single in (0, 1):
+            assert L.pt_ok(h, single)
+            # FP32 entries are rounded once; the products and sums of the walk are double
+            tol = 1e-6 if single else 1e-14
+            for l in range(t):
+                M, Q, G = products(levels, l)
+                live = solvable.astype(float) if l == 0 else np.ones(levels[l].n)
+                b = rng.standard_normal(levels[l].n) * live   # the projected residual is zero on solid cells
+                x = rng.standard_normal(levels[l + 1].n)
+                for up, want, parts, s1 in ((0, M @ b, (1, 2, 3, 8), b), (1, Q @ x + G @ b, (1, 2, 3, 8), x)):
+                    info = (C.c_int * 5)()
+                    L.pt_info(h, single, l if up else l + 1, up, info)
+                    if not (up and l == 0):
+                        assert info[4] == 0 and info[0] % 4 == 0 and info[1] % 4 == 0
+                    if up and not single:
+                        Gl = (G @ sp.diags(live)).tocsr()
+                        Gl.eliminate_zeros()
+                        raw.add((l, int(np.diff(Q.tocsr().indptr).max()), int(np.diff(Gl.indptr).max())))
+                    for p in parts if not (up and l == 0) else (1,):
+                        y = np.empty(len(want))
+                        L.pt_apply(h, single, l if up else l + 1, up, p, s1.ctypes.data, b.ctypes.data, y.ctypes.data)
+                        # a row adds at most a few hundred products of this size
+                        size = max(np.abs(want).max(), np.abs(s1).max(), np.abs(b).max())
+                        assert np.abs(y - want).max() <= tol * 100 * size, (single, l, up, p)
+    finally:
+        L.pt_free(h)
+    return raw
+
+
+@pytest.mark.parametrize("nx,ny,w,i,j,ratio", CHANNELS)
+def test_tables_of_bent_channels(lib, nx, ny, w, i, j, ratio):
+    raw = check(lib, nx, ny, channel(nx, ny, w, i, j), ratio)
+    assert any(l >= 1 and q == 6 and g == 5 for l, q, g in raw), raw   # the mask still has that coarse level
+
+
+@pytest.mark.parametrize("nx,ny,solid,ratio,bc", [
+    (64, 64, False, None, None), (97, 61, True, 16.0, None), (96, 130, True, 16.0, cases.PER),
+    (150, 61, True, None, cases.bcs(right=("pressure_outlet", 0.0, "uniform", 0.3))), (40, 6, False, 16.0, None)])
+def test_tables_of_open_grids(lib, nx, ny, solid, ratio, bc):
+    check(lib, nx, ny, circle(nx, ny) if solid else None, ratio, bc)
