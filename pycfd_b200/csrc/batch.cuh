@@ -2405,6 +2405,14 @@ __global__ void __launch_bounds__(kBThreads) k_b_coarsest(const BProb<T>* __rest
 // preconditioner its FP32 behaviour.
 constexpr int kTailBM = 16, kTailBN = 32, kTailThreads = 256;
 constexpr int kBTailGroup = kTailBN;   // problems per column tile of the tail launch
+// A block's (row tile, column tile) in one word of the map: 12 bits of columns name
+// 131,072 problems of a structure, the 19 above them 8 million rows.
+constexpr int kTailColBits = 12, kTailMaxCols = 1 << kTailColBits;
+__host__ __device__ inline int b_tail_tile(int row_tile, int col_tile) {
+  return (row_tile << kTailColBits) | col_tile;
+}
+__host__ __device__ inline int b_tail_row(int tile) { return tile >> kTailColBits; }
+__host__ __device__ inline int b_tail_col(int tile) { return tile & (kTailMaxCols - 1); }
 
 template <class T> struct TailK;
 template <> struct TailK<float> { static constexpr int KW = 32; };    // K per warp chunk: 4 m16n8k8 steps
@@ -2443,11 +2451,11 @@ __global__ void __launch_bounds__(kTailThreads) k_b_tail(const BProb<T>* __restr
   pdl_begin();   // programmatic dependent launch: the predecessor's results first
   constexpr int KW = TailK<T>::KW;
   constexpr int NW = kTailThreads / 32;
-  const int2 e = map[blockIdx.x];   // (structure, row tile * 64 + column tile)
+  const int2 e = map[blockIdx.x];   // (structure, b_tail_tile)
   const BHier<T>& H = hiers[e.x];
   const int d = H.tail_level;
   const int n = H.tail_n;
-  const int r0 = (e.y >> 6) * kTailBM, ct = e.y & 63;
+  const int r0 = b_tail_row(e.y) * kTailBM, ct = b_tail_col(e.y);
   __shared__ const T* sb[kTailBN];
   __shared__ T* sx[kTailBN];
   __shared__ int any;

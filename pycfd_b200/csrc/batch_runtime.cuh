@@ -50,7 +50,7 @@ struct pycfd_batch {
   std::vector<BMapHost> mapR;              // restriction into d
   std::vector<BMapHost> mapP;              // prolongation into d with P_{d+1}
   std::vector<BMapHost> mapC;              // (problem, -1): coarsest level d of an untailed structure
-  BMapHost mapT;                           // dense tails: (structure, row block x 64 + problem group)
+  BMapHost mapT;                           // dense tails: (structure, b_tail_tile)
   int* sprobs = nullptr;                   // problems grouped by structure
   size_t smem_dense = 0;
   BShared sh{};
@@ -416,8 +416,11 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
       if (H.tail_level == d && H.tail_n > 0) {
         const int rts = (H.tail_n + kTailBM - 1) / kTailBM;
         const int cts = (H.spn + kTailBN - 1) / kTailBN;
+        if (cts > kTailMaxCols)
+          return fail(PCFD_E_UNSUPPORTED, "at most %d problems share a structure with a dense tail",
+                      kTailMaxCols * kTailBN);
         for (int rt = 0; rt < rts; ++rt)
-          for (int c = 0; c < cts; ++c) mt.push_back(make_int2((int)h, rt * 64 + c));
+          for (int c = 0; c < cts; ++c) mt.push_back(make_int2((int)h, b_tail_tile(rt, c)));
       }
       if (B->pats) {
         if (d > H.tail_level) continue;
