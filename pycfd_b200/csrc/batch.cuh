@@ -17,7 +17,9 @@
 // the same problem alone to rounding, and with the reference within the
 // solver tolerance.
 #pragma once
+#include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "boundary.cuh"
 #include "common.cuh"
@@ -2053,6 +2055,7 @@ __global__ void __launch_bounds__(kBThreads, PCFD_BELL_MINB) k_b_ellg(const BPro
 // onto 2 30 -> 22; level 1 up 76 (two launches) -> 37, level 2 up 58 -> 27; level 0 with
 // its last sweep 109 (two launches) -> 68.
 constexpr int kPatGroup = 8;    // problems per block of a coarse level at most
+constexpr int kPatMaxGroups = 1024;   // groups of one structure that a word of the map can name
 constexpr int kPatPart = 12;    // entries a part of a row takes at least
 constexpr int kPatMaxL = 8;     // parts of a row at most
 inline int pat_parts(int K) {
@@ -2098,7 +2101,25 @@ __device__ __forceinline__ void b_pat_rows(const Pat<T>& E, const T* const (&s1)
 }
 
 // Problems per block (gs <= kPatGroup) change no problem's arithmetic, so the engine picks
-// them by what the launch leaves idle (pat_group in the runtime).
+// them by what the launch leaves idle: `usual`, halved while the launch leaves an SM without
+// a block (probs, blocks: problems and row blocks per structure).  A structure whose groups
+// would outnumber the `limit` of the map takes more per block instead, up to `most`.
+inline int b_pick_group(int usual, int most, int limit, int nsm, const std::vector<int>& probs,
+                        const std::vector<int>& blocks) {
+  auto widest = [&](int gs) {
+    int w = 0;
+    for (int n : probs) w = std::max(w, (n + gs - 1) / gs);
+    return w;
+  };
+  int gs = usual;
+  while (gs < most && widest(gs) > limit) gs *= 2;
+  for (; gs > 1; gs /= 2) {
+    long all = 0;
+    for (size_t h = 0; h < probs.size(); ++h) all += (long)blocks[h] * ((probs[h] + gs - 1) / gs);
+    if (all >= nsm || widest(gs / 2) > limit) break;
+  }
+  return gs;
+}
 // The solving members of a block's group, packed to the front; the slots behind them
 // repeat the first member's sources and have no output.
 template <class T, int GS>
@@ -2241,6 +2262,7 @@ __global__ void __launch_bounds__(kBThreads, sizeof(T) == 4 ? 4 : 3) k_b_up(cons
 // problem.  Several rounds of 256 rows for gs <= kUpGroup problems per block, so that the
 // block's sums (two per member) are closed once for 1024 or 2048 rows of each problem.
 constexpr int kUpGroup = 4;
+constexpr int kUpMaxGroups = 4096;   // groups of one structure in a word of that launch's map
 // rounds by rows: 8 from 32768 rows on, 4 below (a structure's own, since they order its sums)
 __host__ __device__ inline int b_up_rounds(int n) { return n >= 32768 ? 8 : 4; }
 template <class T>

@@ -381,25 +381,16 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   if (B->pats) {
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    auto pick = [&](int most, int limit, auto rows) {   // limit: groups per structure the block map can name
-      auto groups = [&](size_t h, int gs) { return (hh[h].spn + gs - 1) / gs; };
-      int gs = most;
-      for (; gs > 1; gs /= 2) {
-        long blocks = 0, widest = 0;
-        for (size_t h = 0; h < leaders.size(); ++h) {
-          blocks += (long)rows(h) * groups(h, gs);
-          widest = std::max<long>(widest, groups(h, gs / 2));
-        }
-        if (blocks >= nsm || widest > limit) break;
-      }
-      return gs;
-    };
-    const int half = sizeof(T) == 4 ? 1 : 2;
-    B->pat_group = pick(kPatGroup / half, 1024, [&](size_t h) {
+    std::vector<int> probs, coarse, fine0;
+    for (size_t h = 0; h < leaders.size(); ++h) {
       const int rpb = kBThreads / hh[h].ld[1];
-      return (keep[h][1].n + rpb - 1) / rpb;
-    });
-    B->up_group = pick(kUpGroup / half, 4096, [&](size_t h) { return pr[leaders[h]].u_chunks; });
+      probs.push_back(hh[h].spn);
+      coarse.push_back((keep[h][1].n + rpb - 1) / rpb);
+      fine0.push_back(pr[leaders[h]].u_chunks);
+    }
+    const int half = sizeof(T) == 4 ? 1 : 2;
+    B->pat_group = b_pick_group(kPatGroup / half, kPatGroup, kPatMaxGroups, nsm, probs, coarse);
+    B->up_group = b_pick_group(kUpGroup / half, kUpGroup, kUpMaxGroups, nsm, probs, fine0);
   }
   B->mapA.assign(B->depth, BMapHost{});
   B->mapR.assign(B->depth, BMapHost{});
@@ -412,7 +403,9 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
       const BHier<T>& H = hh[h];
       const int gs = B->pats ? B->pat_group : B->ell_group;
       const int grps = (H.spn + gs - 1) / gs;
-      if (grps > 1024) return fail(PCFD_E_UNSUPPORTED, "at most %d problems share a structure", 1024 * gs);
+      if (grps > kPatMaxGroups)
+        return fail(PCFD_E_UNSUPPORTED, "at most %d problems share a structure",
+                    kPatMaxGroups * (B->pats ? kPatGroup : gs));
       if (H.tail_level == d && H.tail_n > 0) {
         const int rts = (H.tail_n + kTailBM - 1) / kTailBM;
         const int cts = (H.spn + kTailBN - 1) / kTailBN;

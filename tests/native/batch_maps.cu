@@ -16,4 +16,13 @@ int bm_tail_tile(int row_tile, int col_tile) { return b_tail_tile(row_tile, col_
 int bm_tail_row(int tile) { return b_tail_row(tile); }
 int bm_tail_col(int tile) { return b_tail_col(tile); }
 
+// Problems per block of the pattern products: of a coarse level, or of level 0.
+int bm_pat_group(int single, int level0, int nsm, int n, const int* probs, const int* blocks) {
+  const int half = single ? 1 : 2;
+  const std::vector<int> p(probs, probs + n), b(blocks, blocks + n);
+  return level0 ? b_pick_group(kUpGroup / half, kUpGroup, kUpMaxGroups, nsm, p, b)
+                : b_pick_group(kPatGroup / half, kPatGroup, kPatMaxGroups, nsm, p, b);
+}
+int bm_max_groups(int level0) { return level0 ? kUpMaxGroups : kPatMaxGroups; }
+
 }  // extern "C"

@@ -36,3 +36,10 @@ def test_more_problems_than_64_column_tiles(precision):
     """2100 problems closed by one dense tail: 66 column tiles of 32 problems."""
     from pycfd_b200.batch import BatchOptions
     _equal_problems(20, 2100, BatchOptions(precision=precision, tail_ratio=None))
+
+
+@pytest.mark.parametrize("n,precision", [(20, "fp64"), (10, "fp64"), (10, "mixed")])
+def test_more_problems_than_1024_groups_of_four(n, precision):
+    """4100 problems of one structure: a tail on the 20 x 20 grid, none on the 10 x 10 one."""
+    from pycfd_b200.batch import BatchOptions
+    _equal_problems(n, 4100, BatchOptions(precision=precision, tail_ratio=None if n == 20 else 16.0))
