@@ -50,6 +50,7 @@ struct pycfd_batch {
   std::vector<BMapHost> mapR;              // restriction into d
   std::vector<BMapHost> mapP;              // prolongation into d with P_{d+1}
   std::vector<BMapHost> mapC;              // (problem, -1): coarsest level d of an untailed structure
+  BMapHost mapClose;                       // (problem, -1): untailed structures under the pattern products
   BMapHost mapT;                           // dense tails: (structure, b_tail_tile)
   int* sprobs = nullptr;                   // problems grouped by structure
   size_t smem_dense = 0;
@@ -137,14 +138,15 @@ int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, const PatCycle<T>* c
   const int t = b_closed_at(d);
   if (cyc || (B->coarse == 0 && t < Lv - 1)) {
     const int nt = d->levels[t].n;
-    const double* op = t < Lv - 1 ? d->tail_operator : d->coarsest_inverse;
-    std::vector<T> m((size_t)nt * nt);
-    for (size_t e = 0; e < m.size(); ++e) m[e] = (T)op[e];
-    T* md = nullptr;
-    TRY(upload(B->mem, &md, m.data(), m.size()));
-    H->tail = md;
+    if (t < Lv - 1) {   // an untailed structure is closed per problem (k_b_close)
+      std::vector<T> m((size_t)nt * nt);
+      for (size_t e = 0; e < m.size(); ++e) m[e] = (T)d->tail_operator[e];
+      T* md = nullptr;
+      TRY(upload(B->mem, &md, m.data(), m.size()));
+      H->tail = md;
+      H->tail_n = nt;
+    }
     H->tail_level = t;
-    H->tail_n = nt;
     H->fused = 1;
     for (int l = 1; l <= t; ++l)
       if (!d->levels[l].m_indptr) H->fused = 0;
@@ -396,7 +398,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   B->mapR.assign(B->depth, BMapHost{});
   B->mapP.assign(B->depth, BMapHost{});
   B->mapC.assign(B->depth, BMapHost{});
-  std::vector<int2> mt, m0;
+  std::vector<int2> mt, m0, mclose;
   for (int d = 0; d < B->depth; ++d) {
     std::vector<int2> ma, mr, mp, mc;
     for (size_t h = 0; h < leaders.size(); ++h) {
@@ -417,6 +419,9 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
       }
       if (B->pats) {
         if (d > H.tail_level) continue;
+        if (d == H.tail_level && H.tail_n == 0)
+          for (int i = 0; i < n; ++i)
+            if (hid[i] == (int)h) mclose.push_back(make_int2(i, -1));
         const int nrow = d == 0 ? pr[leaders[h]].g.nx * pr[leaders[h]].g.ny : keep[h][d].n;
         if (d == 0) {
           const int g4 = (H.spn + B->up_group - 1) / B->up_group;
@@ -472,6 +477,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   }
   TRY(upload_map(B, &B->mapT, mt));
   TRY(upload_map(B, &B->map0, m0));
+  TRY(upload_map(B, &B->mapClose, mclose));
   {
     std::vector<int> ord(n);
     for (int i = 0; i < n; ++i) ord[i] = i;
@@ -601,6 +607,9 @@ int b_vcycle(pycfd_batch* B, cudaStream_t st) {
     b_prof(B, 4, st);
     TRY(b_tails<T>(B, st));
     b_prof(B, 4, st);
+    if (B->mapClose.n)
+      BLAUNCH(k_b_close<T>, B->mapClose.n, kBThreads, B->smem_dense, st, probs_of<T>(B), hiers_of<T>(B),
+              B->mapClose.e, B->sh);
     for (int d = D - 1; d >= 1; --d)
       if (B->mapA[d].n)
         BLAUNCH(k_b_up<T>, B->mapA[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapA[d].e, B->sprobs,
