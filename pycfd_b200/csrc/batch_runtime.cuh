@@ -22,10 +22,11 @@ struct pycfd_batch {
   double tol = 1e-10, inner_tol = 1e-4;
   int maxiter = 1000, sweeps = 1, tile_i = 32;
   int coarse = 0;                          // levels >= coarse: one block per problem (0: per level)
-  int fused = 0;                           // down sweep by fused restrictions (every structure has them)
+  int fused = 0;                           // down sweep by fused restrictions (every structure on stored operators has them)
   int fused_from = 1;                      // first level restricted by the fused product (1 or 2)
   int ell_group = kBGroup;                 // problems per block of the coarse-level launches (1 or kBGroup)
-  int pats = 0;                            // the cycle above the tails as pattern products
+  int pats = 0;                            // structures whose cycle above the tail runs as pattern products,
+  int stored = 0;                          // and those on stored operators
   int pat_group = kPatGroup;               // problems per block of their coarse-level launches,
   int up_group = kUpGroup;                 // and of the level-0 up product
   BMapHost map0;                           // level-0 up product: (structure, row block x 4096 + group of kUpGroup)
@@ -41,10 +42,12 @@ struct pycfd_batch {
   int depth = 0;                           // most levels of any problem
   BMapHost fine;                           // every chunk of tiles of every problem
   BMapHost strip;                          // every chunk of warp strips of every problem (solver kernels)
-  BMapHost vstrip;                         // the CG and level-0 sweep kernels: vector chunks where in force
+  BMapHost vstrip;                         // the CG kernels: vector chunks where in force
+  BMapHost sweep0;                         // the level-0 sweeps: vstrip's chunks of the problems on stored operators
   BMapHost halo;                           // every staged tile of every problem (stencil transfers)
   BMapHost pstrip;                         // every chunk of predictor strips of every problem
-  // row-block maps per depth d (problems whose level d runs per level):
+  std::vector<BMapHost> mapDn, mapUp;      // pattern products per depth: (structure, row block x 1024 + group of pat_group)
+  // row-block maps per depth d (problems on stored operators whose level d runs per level):
   // grouped maps per depth d, entries (structure, row block x 1024 + group of ell_group problems):
   std::vector<BMapHost> mapA;              // smoothing/residual with A_d (d >= 1)
   std::vector<BMapHost> mapR;              // restriction into d
@@ -87,7 +90,7 @@ inline int b_closed_at(const pycfd_solver_desc* d) {
 
 // Upload one structure's hierarchy (from the descriptor of its first problem)
 // in storage type T.
-// cyc: the pattern products of its levels (B->pats), which take the place of the ELL blocks.
+// cyc: the pattern products of its levels, which take the place of the ELL blocks (or null).
 template <class T>
 int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, const PatCycle<T>* cyc, BHier<T>* H,
                 std::vector<Level>* keep) {
@@ -190,21 +193,34 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   }
   std::vector<BHier<T>> hh(leaders.size());
   std::vector<std::vector<Level>> keep(leaders.size());
-  // pattern products: one sweep per level and no option asking for another form of the
-  // cycle (the rule reads nothing of the other problems, so that a problem takes the
-  // same route in every split of a batch)
+  // pattern products: one sweep per level, no option asking for another form of the cycle,
+  // and a structure whose rows have few enough patterns; the others keep their stored
+  // operators beside them.  The rule reads nothing of the other structures, so that a
+  // problem takes the same route in every split of a batch.
   std::vector<PatCycle<T>> cyc(leaders.size());
-  B->pats = (B->coarse == 0 && B->sweeps == 1 && B->ell_group == kBGroup && B->fused_from == 1 && !B->stencil_req);
+  std::vector<std::atomic<char>> pat(leaders.size());
   {
+    const bool asked = B->coarse == 0 && B->sweeps == 1 && B->ell_group == kBGroup && B->fused_from == 1 && !B->stencil_req;
     std::vector<std::function<bool()>> tasks;
-    for (size_t h = 0; B->pats && h < leaders.size(); ++h) {
+    for (size_t h = 0; h < leaders.size(); ++h) {
       const pycfd_solver_desc& d = descs[leaders[h]];
-      if (d.n_levels < 2 || d.n_levels > kBMaxLevels || !d.levels || !d.coarsest_inverse ||
-          d.levels[0].n != d.nx * d.ny ||
-          !pat_tasks<T>(d.levels, b_closed_at(&d), true, B->solvers[leaders[h]]->hflags.data(), &cyc[h], &tasks))
-        B->pats = 0;
+      std::vector<std::function<bool()>> own;
+      pat[h] = asked && d.n_levels >= 2 && d.n_levels <= kBMaxLevels && d.levels && d.coarsest_inverse &&
+               d.levels[0].n == d.nx * d.ny &&
+               pat_tasks<T>(d.levels, b_closed_at(&d), true, B->solvers[leaders[h]]->hflags.data(), &cyc[h], &own);
+      for (auto& t : own)
+        if (pat[h]) tasks.push_back([&pat, h, t]() {
+          bool ok = false;
+          try {
+            ok = pat[h] && t();
+          } catch (...) {
+          }
+          if (!ok) pat[h] = 0;
+          return true;
+        });
     }
-    if (B->pats && !run_tasks(tasks)) B->pats = 0;
+    run_tasks(tasks);
+    for (auto& on : pat) (on ? B->pats : B->stored) += 1;
   }
   for (size_t h = 0; h < leaders.size(); ++h) {
     const pycfd_solver_desc& d = descs[leaders[h]];
@@ -214,14 +230,14 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     if (d.n_levels > kBMaxLevels) return fail(PCFD_E_ARG, "at most %d multigrid levels", kBMaxLevels);
     if (d.levels[0].n != d.nx * d.ny) return fail(PCFD_E_ARG, "level 0 must have nx*ny unknowns");
     hh[h] = BHier<T>{};
-    TRY(upload_hier<T>(B, &d, B->pats ? &cyc[h] : nullptr, &hh[h], &keep[h]));
+    TRY(upload_hier<T>(B, &d, pat[h] ? &cyc[h] : nullptr, &hh[h], &keep[h]));
   }
   if (B->smem_dense > 48 * 1024)
     return fail(PCFD_E_UNSUPPORTED, "coarsest level too large for the one-block dense solve");
 
   // per-problem records
   std::vector<BProb<T>> pr(n);
-  std::vector<int2> fine, strip, vstrip, pstrip, halo;
+  std::vector<int2> fine, strip, vstrip, sweep0, pstrip, halo;
   B->nlev.assign(n, 0);
   B->depth = 0;
   int red_rows = 0;
@@ -336,13 +352,17 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     for (int l = 0; l < kBMaxLevels; ++l) P.lv[l] = hh[hid[i]].lv[l];
     for (int c = 0; c < P.chunks; ++c) fine.push_back(make_int2(i, c));
     for (int c = 0; c < P.s_chunks; ++c) strip.push_back(make_int2(i, c));
-    for (int c = 0, nc = P.vec ? P.v_chunks : P.s_chunks; c < nc; ++c) vstrip.push_back(make_int2(i, c));
+    for (int c = 0, nc = P.vec ? P.v_chunks : P.s_chunks; c < nc; ++c) {
+      vstrip.push_back(make_int2(i, c));
+      if (!pat[hid[i]]) sweep0.push_back(make_int2(i, c));
+    }
     for (int c = 0; c < P.h_tiles; ++c) halo.push_back(make_int2(i, c));
     for (int c = 0; c < P.p_chunks; ++c) pstrip.push_back(make_int2(i, c));
   }
   TRY(upload_map(B, &B->fine, fine));
   TRY(upload_map(B, &B->strip, strip));
   TRY(upload_map(B, &B->vstrip, vstrip));
+  TRY(upload_map(B, &B->sweep0, sweep0));
   TRY(upload_map(B, &B->halo, halo));
   TRY(upload_map(B, &B->pstrip, pstrip));
   // problems grouped by structure (the dense tail's block groups)
@@ -364,11 +384,11 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
   // min(coarse, coarsest) on run there and take no per-level blocks.  A problem
   // whose structure has a dense tail at depth t takes the restriction into t
   // and no level below it; the tail blocks cover t.
-  // fused down sweep: every structure closes its cycle with a tail and carries
-  // the fused restrictions above it, one sweep per level
-  B->fused = (B->coarse == 0 && B->sweeps == 1) ? 1 : 0;
+  // fused down sweep: every structure on stored operators closes its cycle with a
+  // tail and carries the fused restrictions above it, one sweep per level
+  B->fused = (B->coarse == 0 && B->sweeps == 1 && B->stored) ? 1 : 0;
   for (size_t h = 0; h < leaders.size(); ++h)
-    if (!hh[h].fused || hh[h].tail_level == 0) B->fused = 0;
+    if (!pat[h] && (!hh[h].fused || hh[h].tail_level == 0)) B->fused = 0;
   // level-0 transfers as stencils: they stand for P_1 and M_1 of the 2 x 2
   // aggregation, so every structure must have that level 1
   B->stencil = (B->stencil_req && B->fused && B->fused_from == 1) ? 1 : 0;
@@ -385,6 +405,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     std::vector<int> probs, coarse, fine0;
     for (size_t h = 0; h < leaders.size(); ++h) {
+      if (!pat[h]) continue;
       const int rpb = kBThreads / hh[h].ld[1];
       probs.push_back(hh[h].spn);
       coarse.push_back((keep[h][1].n + rpb - 1) / rpb);
@@ -394,20 +415,22 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
     B->pat_group = b_pick_group(kPatGroup / half, kPatGroup, kPatMaxGroups, nsm, probs, coarse);
     B->up_group = b_pick_group(kUpGroup / half, kUpGroup, kUpMaxGroups, nsm, probs, fine0);
   }
+  B->mapDn.assign(B->depth, BMapHost{});
+  B->mapUp.assign(B->depth, BMapHost{});
   B->mapA.assign(B->depth, BMapHost{});
   B->mapR.assign(B->depth, BMapHost{});
   B->mapP.assign(B->depth, BMapHost{});
   B->mapC.assign(B->depth, BMapHost{});
   std::vector<int2> mt, m0, mclose;
   for (int d = 0; d < B->depth; ++d) {
-    std::vector<int2> ma, mr, mp, mc;
+    std::vector<int2> ma, mr, mp, mc, mdn, mup;
     for (size_t h = 0; h < leaders.size(); ++h) {
       const BHier<T>& H = hh[h];
-      const int gs = B->pats ? B->pat_group : B->ell_group;
+      const int gs = pat[h] ? B->pat_group : B->ell_group;
       const int grps = (H.spn + gs - 1) / gs;
       if (grps > kPatMaxGroups)
         return fail(PCFD_E_UNSUPPORTED, "at most %d problems share a structure",
-                    kPatMaxGroups * (B->pats ? kPatGroup : gs));
+                    kPatMaxGroups * (pat[h] ? kPatGroup : gs));
       if (H.tail_level == d && H.tail_n > 0) {
         const int rts = (H.tail_n + kTailBM - 1) / kTailBM;
         const int cts = (H.spn + kTailBN - 1) / kTailBN;
@@ -417,7 +440,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
         for (int rt = 0; rt < rts; ++rt)
           for (int c = 0; c < cts; ++c) mt.push_back(make_int2((int)h, b_tail_tile(rt, c)));
       }
-      if (B->pats) {
+      if (pat[h]) {
         if (d > H.tail_level) continue;
         if (d == H.tail_level && H.tail_n == 0)
           for (int i = 0; i < n; ++i)
@@ -433,8 +456,8 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
           for (int rb = 0; rb * (kBThreads / L) < nrow; ++rb)
             for (int g = 0; g < grps; ++g) m.push_back(make_int2((int)h, rb * 1024 + g));
         };
-        rows(mr, H.ld[d]);
-        if (d < H.tail_level) rows(ma, H.lu[d]);
+        rows(mdn, H.ld[d]);
+        if (d < H.tail_level) rows(mup, H.lu[d]);
         continue;
       }
       const int lead = leaders[h];
@@ -470,6 +493,8 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
         add(mr, lres);
       }
     }
+    TRY(upload_map(B, &B->mapDn[d], mdn));
+    TRY(upload_map(B, &B->mapUp[d], mup));
     TRY(upload_map(B, &B->mapA[d], ma));
     TRY(upload_map(B, &B->mapR[d], mr));
     TRY(upload_map(B, &B->mapP[d], mp));
@@ -560,7 +585,7 @@ template <class T, int MODE>
 int b_fine(pycfd_batch* B, int src, int dst, cudaStream_t st) {
   const int id = MODE == FM_LAST ? 2 : MODE == FM_PRE ? 3 : 0;
   b_prof(B, id, st);
-  BLAUNCH((k_b_fine<T, MODE>), B->vstrip.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->vstrip.e, src,
+  BLAUNCH((k_b_fine<T, MODE>), B->sweep0.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->sweep0.e, src,
           dst, B->sh);
   b_prof(B, id, st);
   return 0;
@@ -591,36 +616,12 @@ int b_tails(pycfd_batch* B, cudaStream_t st) {
   return 0;
 }
 
-// One V-cycle from zero on every solving problem, levels in lockstep by depth:
-// z <- M r, with mean(z) and r.z left in each problem's scalar block.  With
-// B->coarse > 0 the levels from there down run in one block per problem.
+// The V-cycle on the stored operators (and every structure's tail), levels in lockstep by
+// depth.  With B->coarse > 0 the levels from there down run in one block per problem.
 template <class T>
-int b_vcycle(pycfd_batch* B, cudaStream_t st) {
+int b_stored_cycle(pycfd_batch* B, cudaStream_t st) {
   const int sw = B->sweeps;
   const int D = B->coarse > 0 ? std::min(B->coarse, B->depth) : B->depth;   // depths run per level
-  if (B->pats) {   // down products, tails, up products: one launch per depth and direction
-    b_prof(B, 4, st);
-    for (int d = 1; d < D; ++d)
-      if (B->mapR[d].n)
-        BLAUNCH(k_b_down<T>, B->mapR[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapR[d].e, B->sprobs,
-                B->pat_group, d, B->sh);
-    b_prof(B, 4, st);
-    TRY(b_tails<T>(B, st));
-    b_prof(B, 4, st);
-    if (B->mapClose.n)
-      BLAUNCH(k_b_close<T>, B->mapClose.n, kBThreads, B->smem_dense, st, probs_of<T>(B), hiers_of<T>(B),
-              B->mapClose.e, B->sh);
-    for (int d = D - 1; d >= 1; --d)
-      if (B->mapA[d].n)
-        BLAUNCH(k_b_up<T>, B->mapA[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapA[d].e, B->sprobs,
-                B->pat_group, d, B->sh);
-    b_prof(B, 4, st);
-    b_prof(B, 2, st);
-    BLAUNCH(k_b_up0<T>, B->map0.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->map0.e, B->sprobs,
-            B->up_group, B->sh);
-    b_prof(B, 2, st);
-    return 0;
-  }
   if (B->fused) {
     // ---- down: b_d = M_d b_{d-1} at every depth from fused_from above each problem's
     // tail (below it the fine sweep and R), then the tails
@@ -702,6 +703,36 @@ int b_vcycle(pycfd_batch* B, cudaStream_t st) {
       std::swap(xf, o);
     }
   }
+  return 0;
+}
+
+// One V-cycle from zero on every solving problem: z <- M r, with mean(z) and r.z left in
+// each problem's scalar block.  The structures on pattern products take one launch per
+// depth and direction around the others' cycle, whose launches do not touch them; the
+// tails of both kinds are one launch.
+template <class T>
+int b_vcycle(pycfd_batch* B, cudaStream_t st) {
+  if (!B->pats) return b_stored_cycle<T>(B, st);
+  b_prof(B, 4, st);
+  for (int d = 1; d < B->depth; ++d)
+    if (B->mapDn[d].n)
+      BLAUNCH(k_b_down<T>, B->mapDn[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapDn[d].e, B->sprobs,
+              B->pat_group, d, B->sh);
+  b_prof(B, 4, st);
+  TRY(B->stored ? b_stored_cycle<T>(B, st) : b_tails<T>(B, st));
+  b_prof(B, 4, st);
+  if (B->mapClose.n)
+    BLAUNCH(k_b_close<T>, B->mapClose.n, kBThreads, B->smem_dense, st, probs_of<T>(B), hiers_of<T>(B), B->mapClose.e,
+            B->sh);
+  for (int d = B->depth - 1; d >= 1; --d)
+    if (B->mapUp[d].n)
+      BLAUNCH(k_b_up<T>, B->mapUp[d].n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->mapUp[d].e, B->sprobs,
+              B->pat_group, d, B->sh);
+  b_prof(B, 4, st);
+  b_prof(B, 2, st);
+  BLAUNCH(k_b_up0<T>, B->map0.n, kBThreads, 0, st, probs_of<T>(B), hiers_of<T>(B), B->map0.e, B->sprobs, B->up_group,
+          B->sh);
+  b_prof(B, 2, st);
   return 0;
 }
 
