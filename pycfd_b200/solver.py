@@ -297,6 +297,8 @@ def native_desc(config, mesh, boundaries, solid, has_obstacle, body_masks, kind,
         if options.coarse_tail and kind is PressureSolver.MGCG:
             tl, top = tail_for(levels, cinv, cfg.mg_sweeps, options.tail_ratio)
         d.tail_level = tl
+        if top is not None:
+            keep.append(top)   # the hierarchy owns it, and may leave its cache before the upload
         d.tail_operator = _lib.cast(top, C.c_double)
         if tl and options.fused_restriction and cfg.mg_sweeps == 1:
             for l, M in enumerate(fused_for(levels, tl), start=1):

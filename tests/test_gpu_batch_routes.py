@@ -52,3 +52,17 @@ def test_a_structure_without_patterns_leaves_the_others_alone(precision, fused):
         assert a[3] == b[3], k
         for p, q in zip(a[:3], b[:3]):
             assert np.array_equal(p, q), k
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_more_structures_than_the_hierarchy_cache_keeps(precision):
+    """Twelve masks of their own in one batch, against each mask alone."""
+    from pycfd_b200.batch import BatchOptions
+    opts = BatchOptions(precision=precision)
+    cfgs = [_cfg(64, 100.0 + 5 * k) for k in range(12)]
+    bodies = [pegs(64, seed=k) for k in range(12)]
+    for k, (a, b) in enumerate(zip(_run(cfgs, bodies, opts),
+                                   (_run(cfgs[k:k + 1], bodies[k:k + 1], opts)[0] for k in range(12)))):
+        assert a[3] == b[3], k
+        for p, q in zip(a[:3], b[:3]):
+            assert np.array_equal(p, q), k
