@@ -217,10 +217,21 @@ struct PatHost {
 // The rows of A (and of B, the second source) as patterns, or false where there are
 // more than the rule allows.  liveA, liveB: entries at columns whose source value is
 // zero by definition are dropped.
-// The rule of one problem alone: at most one pattern per 4 rows on levels over 16384
-// rows, where a row with a pattern of its own would be read uncoalesced; smaller levels
-// stay in L1 and L2 whatever their patterns.  any: no such limit (a batch's groups read
-// an entry once for eight problems, and its problems must not change routes with size).
+// How many patterns pay, measured on masks with nearly as many patterns as rows (one solid
+// cell at a random place of every 4 x 4 block), ms per step.
+// One problem alone: at most one per 4 rows on levels over 16384 rows, where a row with a
+// pattern of its own reads its table uncoalesced (FP64 400x400: 2.3 with the stored
+// operators, 2.6 on patterns; 500x500 2.8 and 2.9); smaller levels stay in L1 and L2 whatever
+// their patterns (256x256 1.63 stored, 1.56 on patterns, 64x64 1.06 and 0.87).
+// any (a batch): no limit but the 65,535 a row can name.  Against the default level-by-level
+// cycle the patterns are always faster (FP64 / mixed, each problem its own mask: 8 of 256x256
+// 8.4 / 8.7 -> 7.3 / 6.6, 24 of 256x256 17.3 / 15.9 -> 15.7 / 14.1, 8 of 400x400 13.6 / 13.6
+// -> 12.8 / 12.4, 64 of 128x128 11.6 / 10.2 -> 11.2 / 9.3).  Against the fused down sweep on
+// stored operators they gain less (one mask 400x400 6.1 / 6.0 -> 4.7 / 5.0, 8 of 256x256 7.6 /
+// 7.5 -> 7.3 / 6.6) and lose up to 6 % where the tables of many such masks outgrow L2 (64 of
+// 128x128 10.6 / 9.0 -> 11.2 / 9.3, 8 of 400x400 12.4 / 11.8 -> 12.8 / 12.4); a limit per
+// structure would not see that, and one per engine would tie a problem's route to its
+// neighbours.
 // up0: the level-0 up product, whose kernels read 6 + 5 entries without padding.
 template <class T>
 bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t* liveB, bool up0, bool any,

@@ -118,3 +118,28 @@ def test_tables_of_bent_channels(lib, nx, ny, w, i, j, ratio):
     (150, 61, True, None, cases.bcs(right=("pressure_outlet", 0.0, "uniform", 0.3))), (40, 6, False, 16.0, None)])
 def test_tables_of_open_grids(lib, nx, ny, solid, ratio, bc):
     check(lib, nx, ny, circle(nx, ny) if solid else None, ratio, bc)
+
+
+def pegs(n, seed=0):
+    """One solid cell at a random place of every 4 x 4 block: nearly every coarse row differs."""
+    rng = np.random.default_rng(seed)
+    solid = np.zeros((n, n), bool)
+    for a in range(0, n - 3, 4):
+        for b in range(0, n - 3, 4):
+            solid[a + rng.integers(3), b + rng.integers(3)] = True
+    return solid
+
+
+def test_tables_of_a_mask_with_a_pattern_per_row(lib):
+    check(lib, 96, 96, pegs(96), 16.0)
+
+
+@pytest.mark.parametrize("n,alone,batch", [(256, True, True), (272, False, True), (560, False, False)])
+def test_how_many_patterns_are_taken(lib, n, alone, batch):
+    """Level 1 has 16384 rows at 256 x 256 (no limit below), 18496 at 272 x 272 (a single
+    problem keeps its stored operators), 78400 at 560 x 560 (more than a row can name)."""
+    levels, t, d, keep, solvable = problem(n, n, pegs(n), 16.0)
+    for any_, want in ((0, alone), (1, batch)):
+        h = lib.pt_build(C.cast(d.levels, C.c_void_p), t, any_, solvable.ctypes.data)
+        assert bool(lib.pt_ok(h, 0)) == bool(lib.pt_ok(h, 1)) == want
+        lib.pt_free(h)
