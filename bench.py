@@ -320,11 +320,10 @@ def batch_cpu_baseline(cfgs, steps=1, warmup=0, workers=None):
                       f"{warmup} untimed step(s), timed together ({wall:.1f} s wall)"}
 
 
-def row_patterns(opts):
-    """Whether a batch of these options runs its V-cycle as row-pattern products, whose
+def row_patterns(b):
+    """Whether every structure of a batch runs its V-cycle as row-pattern products, whose
     level-0 up product is the kernel of kind 2."""
-    return (opts.mg_sweeps == 1 and opts.ell_group == 8 and opts.fused_from == 1
-            and opts.coarse_level == 0 and not opts.stencil_transfer)
+    return all(e.form()["stored_structures"] == 0 for e in getattr(b, "parts", [b]))
 
 
 def kernel_name(kid, patterns):
@@ -431,7 +430,7 @@ def run_batch(args, world, rank, local):
     # roofline: the kernel kind with the largest share of one eager step
     s_bytes = 4 if opts.precision == "mixed" else 8
     cells = np.array([c.nx * c.ny for c in cfgs], dtype=np.float64)
-    prof, pats = {}, row_patterns(opts)
+    prof, pats = {}, row_patterns(b)
     if not args.no_profile:
         for kid in (1, 2, 3, 5, 6):
             kms, kn, kits = b.profile(kid, 1)

@@ -319,6 +319,11 @@ int pycfd_profile_kernel(pycfd_solver* s, int kernel_id);
 /* CTAs of the cooperative launch that runs each CG / MG-PCG solve whole
  * (0: the solver launches one kernel per phase). */
 int pycfd_solver_persistent(pycfd_solver* s, int* ctas);
+/* Which forms the solver's rules chose, form[0..3]: levels whose V-cycle runs as
+ * row-pattern products (0: stored operators), tiles a block of the level-0 product walks
+ * (0: no such product), CTAs of the cluster that runs a Jacobi-CG solve whole (0: one
+ * kernel per phase), solves recorded so far for calls that are not recorded whole. */
+int pycfd_solver_form(pycfd_solver* s, int* form);
 /* No counterpart in the reference (failure detection of the persistent solve).
  * Limit, in nanoseconds, of one grid-barrier wait of the cooperative solve
  * (default 2 s).  A CTA that waits longer sets the launch's error word; every
@@ -497,6 +502,10 @@ int pycfd_batch_initialize(pycfd_batch* b, void* stream);
  * trip (pycfd_get_clock), whose clock reaches t_end or that has taken its
  * max_steps stops; the others go on. */
 int pycfd_batch_step(pycfd_batch* b, int steps, int record, void* stream);
+/* Which forms the engine's rules chose, form[0..3]: structures whose V-cycle runs as
+ * row-pattern products, structures on stored operators, problems per block of the
+ * coarse-level launches, and of the level-0 product (0: no such product). */
+int pycfd_batch_form(pycfd_batch* b, int* form);
 /* Problem i's single-problem handle (clock, stats, reductions; not for stepping). */
 pycfd_solver* pycfd_batch_problem(pycfd_batch* b, int i);
 /* Per-problem arrays of n: frozen (0 running, 1 stopped by a health flag,

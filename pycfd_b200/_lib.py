@@ -30,6 +30,7 @@ EXPORTS = (
     "pycfd_history_read",
     "pycfd_step_host", "pycfd_get_stats", "pycfd_reduce_fields", "pycfd_face_lists", "pycfd_rasterize", "pycfd_adjoint_apply",
     "pycfd_reduce_fields_noalloc", "pycfd_profile_kernel", "pycfd_solver_persistent",
+    "pycfd_solver_form", "pycfd_batch_form",
     "pycfd_solver_set_wait_limit", "pycfd_solve_trace", "pycfd_launch_count",
     "pycfd_profile_read", "pycfd_batch_create", "pycfd_batch_destroy", "pycfd_batch_initialize",
     "pycfd_batch_step", "pycfd_batch_problem", "pycfd_batch_status", "pycfd_batch_launches",
@@ -158,6 +159,8 @@ def load(path: str = LIB_PATH):
         "pycfd_get_stats": (C.c_int, [vp, C.POINTER(Stats), vp]),
         "pycfd_profile_kernel": (C.c_int, [vp, C.c_int]),
         "pycfd_solver_persistent": (C.c_int, [vp, C.POINTER(C.c_int)]),
+        "pycfd_solver_form": (C.c_int, [vp, C.POINTER(C.c_int)]),
+        "pycfd_batch_form": (C.c_int, [vp, C.POINTER(C.c_int)]),
         "pycfd_solver_set_wait_limit": (C.c_int, [vp, C.c_ulonglong]),
         "pycfd_solve_trace": (C.c_int, [vp, C.c_int, C.POINTER(C.c_ulonglong), C.c_int, vp]),
         "pycfd_launch_count": (C.c_longlong, []),

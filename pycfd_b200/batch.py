@@ -413,6 +413,15 @@ class BatchedSolver:
         return {"frozen": np.array(fr[:]), "steps": np.array(st[:]), "iterations": np.array(it[:]),
                 "status": np.array(ss[:]), "t": np.array(t[:]), "dt": np.array(dt[:])}
 
+    def form(self) -> dict:
+        """Which forms the engine's rules chose: ``pattern_structures`` and
+        ``stored_structures`` (their V-cycle as row-pattern products, or on stored
+        operators), ``group`` and ``up_group`` (problems per block of the coarse-level
+        launches and of the level-0 product)."""
+        out = (C.c_int * 4)()
+        _lib.check(self._L.pycfd_batch_form(self._h, out))
+        return dict(zip(("pattern_structures", "stored_structures", "group", "up_group"), out[:]))
+
     def field(self, k: int) -> FlowField:
         """Problem ``k``'s state (the batch's own tensors; copy to keep a snapshot)."""
         st = self.status()

@@ -1085,6 +1085,15 @@ int pycfd_batch_capped(pycfd_batch* B, int* capped, void* stream) {
   return 0;
 }
 
+int pycfd_batch_form(pycfd_batch* B, int* form) {
+  if (!B || !form) return fail(PCFD_E_ARG, "bad arguments");
+  form[0] = B->pats;
+  form[1] = B->stored;
+  form[2] = B->pats ? B->pat_group : B->ell_group;
+  form[3] = B->pats ? B->up_group : 0;
+  return 0;
+}
+
 pycfd_solver* pycfd_batch_problem(pycfd_batch* B, int i) {
   if (!B || i < 0 || i >= B->n) return nullptr;
   return B->solvers[i];

@@ -337,6 +337,13 @@ inline PatLaunch pat_launch(const Pat<T>& E, long threads, bool parts) {
   p.grid = dim3((E.ny_r + tj - 1) / tj, (rx + ti - 1) / ti);
   return p;
 }
+// Grid of the level-0 up product: one wave of blocks, each walking `rounds` tiles along x.
+template <class T>
+inline dim3 pat_up0_grid(const Pat<T>& E, long threads, int blocks, int* rounds) {
+  const PatLaunch q = pat_launch(E, threads, false);
+  *rounds = (int)(((long)q.grid.x * q.grid.y + blocks - 1) / blocks);
+  return dim3(q.grid.x, (q.grid.y + *rounds - 1) / *rounds);
+}
 template <class T>
 __device__ __forceinline__ int pat_base_ij(const Pat<T>& E, int i, int j) {
   return E.base == PB_COARSER ? (i >> (E.fx - 1)) * E.ny_c + (j >> (E.fy - 1))

@@ -530,10 +530,8 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
     prof_mark(s, 2, stream);
     {
       const Pat<T>& E = patUp<T>(s)[0];
-      const PatLaunch q = pat_launch(E, s->pat_threads, false);
-      const long tiles = (long)q.grid.x * q.grid.y;
-      const int rounds = (int)((tiles + s->pat_blocks - 1) / s->pat_blocks);   // one wave of blocks
-      const dim3 grid(q.grid.x, (q.grid.y + rounds - 1) / rounds);
+      int rounds = 1;
+      const dim3 grid = pat_up0_grid(E, s->pat_threads, s->pat_blocks, &rounds);
       pdl_launch(s, E.f65 ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds,
                  (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, s->singular, (const double*)s->S, z_out, s->zpart);
       s->nz = (int)(grid.x * grid.y);
@@ -2220,6 +2218,17 @@ int pycfd_solver_set_wait_limit(pycfd_solver* s, unsigned long long ns) {
 int pycfd_solver_persistent(pycfd_solver* s, int* ctas) {
   if (!s || !ctas) return fail(PCFD_E_ARG, "bad arguments");
   *ctas = s->persistent;
+  return 0;
+}
+
+int pycfd_solver_form(pycfd_solver* s, int* form) {
+  if (!s || !form) return fail(PCFD_E_ARG, "bad arguments");
+  int rounds = 0;
+  if (!s->pup.empty()) pat_up0_grid(s->pup[0], s->pat_threads, s->pat_blocks, &rounds);
+  form[0] = s->pup.empty() ? 0 : s->tail_level;
+  form[1] = rounds;
+  form[2] = s->cl_ctas;
+  form[3] = (int)s->solve_graphs.size();
   return 0;
 }
 

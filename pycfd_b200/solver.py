@@ -480,6 +480,15 @@ class ProjectionSolver:
         #: CTAs of the cooperative launch of each CG / MG-PCG solve (0: per-phase kernels)
         self._persistent = int(ctas.value)
 
+    def form(self) -> dict:
+        """Which forms the solver's rules chose: ``pattern_levels`` (levels whose V-cycle
+        runs as row-pattern products, 0: stored operators), ``up_tiles`` (tiles a block of
+        the level-0 product walks), ``cluster_ctas`` (of the launch that runs a Jacobi-CG
+        solve whole, 0: one kernel per phase), ``recorded_solves``."""
+        out = (C.c_int * 4)()
+        _lib.check(self._L.pycfd_solver_form(self._h, out))
+        return dict(zip(("pattern_levels", "up_tiles", "cluster_ctas", "recorded_solves"), out[:]))
+
     def set_wait_limit(self, seconds: float) -> None:
         """Limit of one grid-barrier wait of the persistent solve (default 2 s).  A
         wait that runs out ends the solve with a ``RuntimeError``; the solver stays
