@@ -340,7 +340,8 @@ int pycfd_solver_set_wait_limit(pycfd_solver* s, unsigned long long ns);
  * most cap words. */
 int pycfd_solve_trace(pycfd_solver* s, int enable, unsigned long long* out, int cap, void* stream);
 /* Kernel launches issued by this library so far (eager launches; a recorded
- * step counts its launches once, when it is recorded). */
+ * step counts its launches once, when it is recorded; a recorded solve with every
+ * replay, its loop's launches once pycfd_get_stats has read the iterations). */
 long long pycfd_launch_count(void);
 int pycfd_profile_read(pycfd_solver* s, double* total_ms, int* launches, void* stream);
 

@@ -802,9 +802,9 @@ int b_solve_fp64(pycfd_batch* B, cudaStream_t st) {
   };
   if (B->capturing) {
     TRY(b_loop_open(st, B->aux, ctl));
-    const long long l0 = g_launches.load();
+    const long long l0 = t_launches;
     TRY(pass(B->aux));
-    B->cg_body_launches = g_launches.load() - l0;
+    B->cg_body_launches = t_launches - l0;
     TRY(b_loop_close(B->aux));
   } else {
     for (int guard = 0; guard <= B->maxiter; ++guard) {
@@ -845,17 +845,17 @@ int b_solve_mixed(pycfd_batch* B, cudaStream_t st) {
   };
   if (B->capturing) {
     TRY(b_loop_open(st, B->aux, outer));
-    const long long l0 = g_launches.load();
+    const long long l0 = t_launches;
     cudaGraph_t body = nullptr;
     TRY(b_loop_handle(B->aux, &body, &inner));
     BLAUNCH(k_b_ir_arm<T>, 1, kBThreads, 0, B->aux, P, B->n, B->sh, inner);
     TRY(b_loop_open(B->aux, B->aux2, inner));
-    const long long l1 = g_launches.load();
+    const long long l1 = t_launches;
     TRY(inner_pass(B->aux2));
-    B->cg_body_launches = g_launches.load() - l1;
+    B->cg_body_launches = t_launches - l1;
     TRY(b_loop_close(B->aux2));
     TRY(refine(B->aux));
-    B->ir_body_launches = g_launches.load() - l0 - B->cg_body_launches;
+    B->ir_body_launches = t_launches - l0 - B->cg_body_launches;
     TRY(b_loop_close(B->aux));
   } else {
     for (int g1 = 0; g1 <= kIrMaxPassesB + 1; ++g1) {
@@ -1033,7 +1033,7 @@ int pycfd_batch_step(pycfd_batch* B, int steps, int record, void* stream) {
     if (!B->rec) CU(cudaStreamCreateWithFlags(&B->rec, cudaStreamNonBlocking));
     CU(cudaStreamBeginCapture(B->rec, cudaStreamCaptureModeThreadLocal));
     B->capturing = true;
-    const long long l0 = g_launches.load();
+    const long long l0 = t_launches;
     int rc = b_dispatch_step(B, B->rec);
     B->capturing = false;
     cudaGraph_t graph = nullptr;
@@ -1043,7 +1043,7 @@ int pycfd_batch_step(pycfd_batch* B, int steps, int record, void* stream) {
       return rc;
     }
     if (ec != cudaSuccess) return fail(PCFD_E_CUDA, "batch step capture failed: %s", cudaGetErrorString(ec));
-    const long long rec_total = g_launches.load() - l0;
+    const long long rec_total = t_launches - l0;
     // 3 solves per step: each solve's loop bodies counted once while recording
     B->fixed_launches = rec_total - 3 * (B->cg_body_launches + B->ir_body_launches);
     CU(cudaGraphInstantiate(&B->exec, graph, 0));

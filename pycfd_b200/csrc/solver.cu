@@ -51,11 +51,17 @@ static int fail(int code, const char* fmt, ...) {
   } while (0)
 
 // Every kernel launch is followed by exactly one CHECK_LAUNCH, which also
-// counts it (pycfd_launch_count) -- recorded launches count once, when recorded.
+// counts it (pycfd_launch_count) -- recorded launches count once, when recorded.  What a
+// recording holds is counted per thread, beside other threads' launches.
 static std::atomic<long long> g_launches{0};
+static thread_local long long t_launches = 0;
+static inline void count_launches(long long n) {
+  g_launches.fetch_add(n);
+  t_launches += n;
+}
 #define CHECK_LAUNCH()          \
   do {                          \
-    g_launches.fetch_add(1);    \
+    count_launches(1);          \
     CU(cudaGetLastError());     \
   } while (0)
 #define TRY(x)             \
@@ -212,6 +218,7 @@ struct pycfd_solver {
   };
   std::vector<SolveGraph> solve_graphs;
   int host_solves = 0;          // solves run with the loop on the host so far
+  bool unrecorded = false;      // a solve could not be recorded: the loop stays on the host
   long long body_launches = 0;  // launches of the loop body recorded last
   long long replay_body = 0;    // ... of the replays whose iterations are not counted yet
 
@@ -473,7 +480,7 @@ int launch_coarse_cluster(pycfd_solver* s, int lc, const T* res_in, T** out, cud
   cfg.numAttrs = 1;
   prof_mark(s, 4, stream);
   CU(cudaLaunchKernelEx(&cfg, k_coarse_cycle<T>, t));
-  g_launches.fetch_add(1);
+  count_launches(1);
   prof_mark(s, 4, stream);
   // where x_lc ends: the first sweep writes xa; each further sweep swaps
   LevelBuf<T>& B = lvB<T>(s->lv[lc]);
@@ -896,9 +903,9 @@ int solve_mixed(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
       if (!s->aux2) CU(cudaStreamCreateWithFlags(&s->aux2, cudaStreamNonBlocking));
       CU(cudaStreamBeginCaptureToGraph(s->aux2, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                        cudaStreamCaptureModeRelaxed));
-      const long long l0 = g_launches.load();
+      const long long l0 = t_launches;
       TRY(inner_pass(s->aux2));
-      s->body_launches = g_launches.load() - l0;
+      s->body_launches = t_launches - l0;
       cudaGraph_t dummy = nullptr;
       CU(cudaStreamEndCapture(s->aux2, &dummy));
     }
@@ -1175,9 +1182,9 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
       TRY(launch_cg_cluster(s, x, stream));
     } else if (cap) {
       TRY(loop_open(s, stream, &L));
-      const long long l0 = g_launches.load();
+      const long long l0 = t_launches;
       TRY(pass(s->aux));
-      s->body_launches = g_launches.load() - l0;
+      s->body_launches = t_launches - l0;
       TRY(loop_close(s));
     } else {
       for (;;) {
@@ -1212,9 +1219,9 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
       };
       if (cap) {
         TRY(loop_open(s, stream, &L));
-        const long long l0 = g_launches.load();
+        const long long l0 = t_launches;
         TRY(cycle(s->aux));
-        s->body_launches = g_launches.load() - l0;
+        s->body_launches = t_launches - l0;
         TRY(loop_close(s));
       } else {
         for (;;) {
@@ -1260,56 +1267,75 @@ int solve_prepared(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream)
   return 0;
 }
 
+int solve_direct(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
+  return s->precision == PCFD_MIXED ? solve_mixed(s, x, has_x0, stream) : solve_prepared(s, x, has_x0, stream);
+}
+
+// Ends what is still being recorded on a stream of the solver's own after an error.
+void drop_capture(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaGraph_t g = nullptr;
+  if (stream && cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+    cudaStreamEndCapture(stream, &g);   // a loop's body: its graph belongs to the parent
+}
+
+// Records the solve into e.  An error leaves nothing recorded and nothing behind.
+int record_solve(pycfd_solver* s, pycfd_solver::SolveGraph* e) {
+  if (!s->aux) CU(cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking));
+  if (!s->rec) CU(cudaStreamCreateWithFlags(&s->rec, cudaStreamNonBlocking));
+  CU(cudaStreamBeginCapture(s->rec, cudaStreamCaptureModeThreadLocal));
+  s->capturing = true;
+  s->body_launches = 0;
+  const long long l0 = t_launches;
+  int rc = solve_direct(s, e->x, e->has_x0, s->rec);
+  s->capturing = false;
+  const long long all = t_launches - l0;
+  count_launches(-all);   // counted with every replay
+  if (rc) {
+    drop_capture(s->aux2);
+    drop_capture(s->aux);
+  }
+  const cudaError_t ec = cudaStreamEndCapture(s->rec, &e->graph);
+  if (!rc && ec != cudaSuccess) rc = fail(PCFD_E_CUDA, "solve capture failed: %s", cudaGetErrorString(ec));
+  if (!rc && cudaGraphInstantiate(&e->exec, e->graph, 0) != cudaSuccess)
+    rc = fail(PCFD_E_CUDA, "solve recording failed: %s", cudaGetErrorString(cudaGetLastError()));
+  if (rc && e->graph) cudaGraphDestroy(e->graph);
+  e->body = s->body_launches;
+  e->fixed = all - e->body;
+  return rc;
+}
+
 // The solve of a call that is not recorded whole.  Its iteration loop runs on the host --
 // one read of the done flag per pass -- for a solver's first solves, and as a recorded
 // solve with the loop on the device from then on, so that a solver used for a few solves
 // does not pay for the recording (about two steps' worth of solves; 128x128 MG-PCG step
 // 1.58 -> 1.20 ms).  Recorded solves are kept per iterate buffer (the solver's own) and
-// warm start.  Per-kernel timing needs the host loop.
+// warm start.  Per-kernel timing needs the host loop, and so does a solver whose solve
+// could not be recorded (device memory for the graph): it stays on the host loop.
 constexpr int kHostSolves = 6;
 int solve_rhs(pycfd_solver* s, double* x, bool has_x0, cudaStream_t stream) {
-  auto direct = [&](cudaStream_t st) {
-    return s->precision == PCFD_MIXED ? solve_mixed(s, x, has_x0, st) : solve_prepared(s, x, has_x0, st);
-  };
   if (s->capturing || s->prof_id || s->persistent || s->cl_ctas || s->solver_kind == PCFD_SOLVER_JACOBI ||
-      s->solver_kind == PCFD_SOLVER_SOR || s->host_solves < kHostSolves) {
+      s->solver_kind == PCFD_SOLVER_SOR || s->unrecorded || s->host_solves < kHostSolves) {
     if (!s->capturing) ++s->host_solves;
-    return direct(stream);
+    return solve_direct(s, x, has_x0, stream);
   }
   pycfd_solver::SolveGraph* hit = nullptr;
   for (auto& e : s->solve_graphs)
     if (e.x == x && e.has_x0 == has_x0) hit = &e;
   if (!hit) {
-    if (!s->aux) CU(cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking));
-    if (!s->rec) CU(cudaStreamCreateWithFlags(&s->rec, cudaStreamNonBlocking));
     pycfd_solver::SolveGraph e{};
     e.x = x;
     e.has_x0 = has_x0;
-    CU(cudaStreamBeginCapture(s->rec, cudaStreamCaptureModeThreadLocal));
-    s->capturing = true;
-    s->body_launches = 0;
-    const long long l0 = g_launches.load();
-    const int rc = direct(s->rec);
-    s->capturing = false;
-    const long long all = g_launches.load() - l0;
-    const cudaError_t ec = cudaStreamEndCapture(s->rec, &e.graph);
-    if (rc) {
-      if (e.graph) cudaGraphDestroy(e.graph);
-      return rc;
+    if (record_solve(s, &e)) {
+      s->unrecorded = true;
+      cudaGetLastError();
+      return solve_direct(s, x, has_x0, stream);
     }
-    if (ec != cudaSuccess) return fail(PCFD_E_CUDA, "solve capture failed: %s", cudaGetErrorString(ec));
-    if (cudaGraphInstantiate(&e.exec, e.graph, 0) != cudaSuccess) {
-      cudaGraphDestroy(e.graph);
-      return fail(PCFD_E_CUDA, "solve recording failed: %s", cudaGetErrorString(cudaGetLastError()));
-    }
-    g_launches.fetch_sub(all);   // counted below, with every replay
-    e.body = s->body_launches;
-    e.fixed = all - e.body;
     s->solve_graphs.push_back(e);
     hit = &s->solve_graphs.back();
   }
   CU(cudaGraphLaunch(hit->exec, stream));
-  g_launches.fetch_add(hit->fixed);
+  count_launches(hit->fixed);
   s->replay_body = hit->body;    // times the iterations, once they are read (pycfd_get_stats)
   return 0;
 }
@@ -2045,7 +2071,7 @@ int record_gated_step(pycfd_solver* s, const double* u0, const double* v0, doubl
     if (cudaGetLastError() != cudaSuccess) rc = fail(PCFD_E_CUDA, "stats launch failed");
     k_history_append<<<1, 32, 0, s->gate>>>(s->S, s->I, s->hist, kHistRows, c);
     if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(PCFD_E_CUDA, "history launch failed");
-    g_launches.fetch_add(2);
+    count_launches(2);
   }
   cudaGraph_t body = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(s->gate, &body);
@@ -2095,11 +2121,11 @@ int pycfd_step_adaptive(pycfd_solver* s, const double* u0, const double* v0, dou
     pdl_launch(s, k_field_stats, std::min(s->g.nx + 3, kMaxRedBlocks), kRedThreads, 0, s->rec, 
         u0, v0, nullptr, nullptr, nullptr, s->solid, s->g, s->rb(), s->S);
     if (cudaGetLastError() != cudaSuccess) rc = fail(PCFD_E_CUDA, "stats launch failed");
-    g_launches.fetch_add(1);
+    count_launches(1);
     if (!c.history) {
       pdl_launch(s, k_adaptive_dt, 1, 32, 0, s->rec, s->S, s->I, c);
       if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(PCFD_E_CUDA, "dt launch failed");
-      g_launches.fetch_add(1);
+      count_launches(1);
       if (!rc) rc = step_impl(s, u0, v0, u, v, p, s->rec);
     } else if (!rc) {
       // gated step: [gate] -> IF { step, statistics of the new state, history row }
@@ -2414,7 +2440,7 @@ int pycfd_get_stats(pycfd_solver* s, pycfd_stats* o, void* stream) {
     o->body_fy[b] = s->hS[S_BODY_FY + b];
   }
   o->ir_iterations = s->hI[I_IR_IT];
-  if (s->replay_body) g_launches.fetch_add(s->replay_body * s->hI[I_TOTAL_IT]);   // replayed solves of this call
+  if (s->replay_body) count_launches(s->replay_body * s->hI[I_TOTAL_IT]);   // replayed solves of this call
   s->replay_body = 0;
   return 0;
 }

@@ -103,3 +103,37 @@ def test_groups_of_a_batch(precision, count, group, up):
     for x, y in zip(fields, fields_g):
         for p, q in zip(x, y):
             assert np.abs(p - q).max() <= 1e-8 * max(np.abs(f).max() for f in y)
+
+
+def test_launch_counts_of_recorded_solves_beside_other_threads():
+    """What a recording holds is counted apart from the launches that other threads make
+    meanwhile: solves on four threads count what they count one after another."""
+    import threading
+    from pycfd_b200 import _lib
+    L = _lib.load()
+    sizes = [(64, 64), (96, 64), (80, 112), (128, 128)]
+    rhs = [np.random.default_rng(k).standard_normal(n) for k, n in enumerate(sizes)]
+
+    def work(k, s, barrier=None):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            if barrier:
+                barrier.wait()
+            for _ in range(12):
+                s.pressure_solver.solve(rhs[k])
+
+    def total(threads):
+        solvers = [_solver(_cfg(*n)) for n in sizes]
+        torch.cuda.synchronize()
+        n0 = L.pycfd_launch_count()
+        if threads:
+            b = threading.Barrier(len(sizes))
+            ts = [threading.Thread(target=work, args=(k, s, b)) for k, s in enumerate(solvers)]
+            [t.start() for t in ts]
+            [t.join() for t in ts]
+        else:
+            [work(k, s) for k, s in enumerate(solvers)]
+        assert all(s.form()["recorded_solves"] == 1 for s in solvers)
+        return L.pycfd_launch_count() - n0
+
+    one_by_one = total(False)
+    assert one_by_one > 0 and total(True) == one_by_one
