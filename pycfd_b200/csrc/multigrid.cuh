@@ -337,6 +337,9 @@ inline PatLaunch pat_launch(const Pat<T>& E, long threads, bool parts) {
   p.grid = dim3((E.ny_r + tj - 1) / tj, (rx + ti - 1) / ti);
   return p;
 }
+// Whether that launch is one the GPU takes: 65,535 tiles along x at most (524,280 rows of a
+// grid a few cells wide, whose level stays on stored operators).
+inline bool pat_fits(const PatLaunch& p) { return p.grid.y <= 65535u; }
 // Grid of the level-0 up product: one wave of blocks, each walking `rounds` tiles along x.
 template <class T>
 inline dim3 pat_up0_grid(const Pat<T>& E, long threads, int blocks, int* rounds) {

@@ -1023,6 +1023,10 @@ bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
   if (!pat_tasks<double>(d->levels, t, false, s->hflags.data(), &cd, &tasks)) return false;
   if (mixed && !pat_tasks<float>(d->levels, t, false, s->hflags.data(), &cf, &tasks)) return false;
   if (!run_tasks(tasks)) return false;
+  for (int l = 1; l <= t; ++l)
+    if (!pat_fits(pat_launch(cd.dn[l].v, s->pat_threads, true)) ||
+        (l < t && !pat_fits(pat_launch(cd.up[l].v, s->pat_threads, true))))
+      return false;
   auto keep = [&](auto& c, auto& dn, auto& up) -> int {
     dn.resize(t + 1);
     up.resize(t + 1);

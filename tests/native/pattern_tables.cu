@@ -12,6 +12,7 @@
 
 #include "../../include/pycfd_b200.h"
 #include "../../pycfd_b200/csrc/common.cuh"
+#include "../../pycfd_b200/csrc/multigrid.cuh"
 #include "../../pycfd_b200/csrc/pattern.cuh"
 
 using namespace pcfd;
@@ -118,6 +119,15 @@ void pt_apply(void* h, int single, int l, int up, int parts, const double* s1, c
   const Cycle& c = *(Cycle*)h;
   if (single) apply<float>(pick(c.f, l, up).v, pick(c.f, l, up), up && l == 0, parts, s1, s2, y);
   else apply<double>(pick(c.d, l, up).v, pick(c.d, l, up), up && l == 0, parts, s1, s2, y);
+}
+
+// Whether the launch of a product over nx x ny rows of K entries fits the GPU's grid.
+int pt_fits(int nx, int ny, int K) {
+  Pat<double> E{};
+  E.n = nx * ny;
+  E.ny_r = ny;
+  E.K = K;
+  return pat_fits(pat_launch(E, 592 * 256, true));
 }
 
 }  // extern "C"

@@ -143,3 +143,10 @@ def test_how_many_patterns_are_taken(lib, n, alone, batch):
         h = lib.pt_build(C.cast(d.levels, C.c_void_p), t, any_, solvable.ctypes.data)
         assert bool(lib.pt_ok(h, 0)) == bool(lib.pt_ok(h, 1)) == want
         lib.pt_free(h)
+
+
+@pytest.mark.parametrize("nx,ny,fits", [(524280, 2, True), (524281, 2, False), (2, 524281, True), (600000, 4, False),
+                                        (8192, 8192, True), (20000, 1, True)])
+def test_grids_of_the_products(lib, nx, ny, fits):
+    """8 rows of tiles along x per block: more than 65,535 blocks along x are not launched."""
+    assert bool(lib.pt_fits(nx, ny, 24)) == fits
