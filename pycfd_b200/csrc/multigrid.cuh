@@ -321,10 +321,19 @@ __global__ void k_ell_prolong0_wb(Ell<T> P, B bf, const uint8_t* __restrict__ fl
 #define PCFD_PAT_MINB 4
 #endif
 constexpr int kPatMaxParts = 32;
-// Rows along y of a tile.
-__host__ __device__ inline int pat_tile_j(int L) { return L <= 8 ? 32 : 256 / L; }
+// Rows along y of a tile: 32, fewer where a block has fewer rows than that or the grid is no
+// more than half as wide.  A power of two, as its logarithm.  Solves in ms, tiles of 32 at any
+// width (most of their lanes idle) -> these, with the stored operators in brackets: FP64
+// 100000x4 3.47 -> 1.33 (2.11), 20000x4 1.12 -> 0.61 (0.93), 20000x16 1.32 -> 1.05 (1.36);
+// mixed 100000x4 5.89 -> 2.02 (3.36).
+inline int pat_tile_sh(int L, int ny) {
+  int sh = 5;
+  while ((1 << sh) * L > 256) --sh;
+  while (sh > 0 && (1 << (sh - 1)) >= ny) --sh;
+  return sh;
+}
 struct PatLaunch {
-  int L = 1;
+  int L = 1, sh = 5;   // parts of a row; logarithm of the rows along y
   dim3 grid;
 };
 // Parts: about two units each, within the resident threads of the GPU.
@@ -333,17 +342,19 @@ inline PatLaunch pat_launch(const Pat<T>& E, long threads, bool parts) {
   PatLaunch p;
   const int K = E.K + E.K2, rx = E.n / E.ny_r;
   while (parts && p.L < kPatMaxParts && K >= 2 * kPatUnit * p.L && (long)E.n * p.L * 2 <= threads) p.L *= 2;
-  const int tj = pat_tile_j(p.L), ti = 256 / p.L / tj;
+  p.sh = pat_tile_sh(p.L, E.ny_r);
+  const int tj = 1 << p.sh, ti = 256 / p.L / tj;
   p.grid = dim3((E.ny_r + tj - 1) / tj, (rx + ti - 1) / ti);
   return p;
 }
-// Whether that launch is one the GPU takes: 65,535 tiles along x at most (524,280 rows of a
-// grid a few cells wide, whose level stays on stored operators).
+// Whether that launch is one the GPU takes: 65,535 tiles along x at most (524,280 rows at 32
+// along y; a longer level stays on stored operators).
 inline bool pat_fits(const PatLaunch& p) { return p.grid.y <= 65535u; }
 // Grid of the level-0 up product: one wave of blocks, each walking `rounds` tiles along x.
 template <class T>
-inline dim3 pat_up0_grid(const Pat<T>& E, long threads, int blocks, int* rounds) {
+inline dim3 pat_up0_grid(const Pat<T>& E, long threads, int blocks, int* rounds, int* sh) {
   const PatLaunch q = pat_launch(E, threads, false);
+  *sh = q.sh;
   *rounds = (int)(((long)q.grid.x * q.grid.y + blocks - 1) / blocks);
   return dim3(q.grid.x, (q.grid.y + *rounds - 1) / *rounds);
 }
@@ -354,15 +365,25 @@ __device__ __forceinline__ int pat_base_ij(const Pat<T>& E, int i, int j) {
                               : i * E.ny_r + j;
 }
 
+// A thread's part and row (i, j) in a launch of L parts and tiles 1 << sh rows wide; returns
+// the row's place in the block.
+__host__ __device__ __forceinline__ int pat_thread(int t, int bx, int by, int L, int sh, int* part, int* i, int* j) {
+  const int rpb = 256 / L, ti = rpb >> sh;
+  *part = t / rpb;
+  const int rl = t - *part * rpb;
+  *i = by * ti + (rl >> sh);
+  *j = (bx << sh) + (rl & ((1 << sh) - 1));
+  return rl;
+}
+
 // y = E s1 (+ second source s2).  FROM_R: the source of a down product is the CG residual
 // less its fluid mean.
 template <class T, bool FROM_R>
 __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
-    k_pat(Pat<T> E, int L, const T* __restrict__ s1, const T* __restrict__ s2, const double* __restrict__ S,
+    k_pat(Pat<T> E, int L, int sh, const T* __restrict__ s1, const T* __restrict__ s2, const double* __restrict__ S,
           int singular, T* __restrict__ y) {
-  const int tj = pat_tile_j(L), rpb = 256 / L, ti = rpb / tj;
-  const int part = (int)threadIdx.x / rpb, rl = (int)threadIdx.x - part * rpb;
-  const int i = (int)blockIdx.y * ti + rl / tj, j = (int)blockIdx.x * tj + rl % tj;
+  int part, i, j;
+  const int rl = pat_thread((int)threadIdx.x, (int)blockIdx.x, (int)blockIdx.y, L, sh, &part, &i, &j), rpb = 256 / L;
   const int row = i * E.ny_r + j;
   const bool ok = j < E.ny_r && row < E.n;
   // the tables, which no kernel writes, ahead of the wait for the predecessor
@@ -393,13 +414,13 @@ __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
 // and r.z for the projected z and rho; a block walks `rounds` tiles along x.
 template <class T, bool F65>
 __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
-    k_pat_up0(Pat<T> E, int rounds, const T* __restrict__ x1, const T* __restrict__ r,
+    k_pat_up0(Pat<T> E, int rounds, int sh, const T* __restrict__ x1, const T* __restrict__ r,
               const uint8_t* __restrict__ flags, int singular, const double* __restrict__ S, T* __restrict__ z,
               double* __restrict__ zpart) {
-  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
-  const int j = (int)blockIdx.x * 32 + lane, nx = E.n / E.ny_r;
-  const int i1 = min(nx, ((int)blockIdx.y + 1) * rounds * 8);
-  int i = (int)blockIdx.y * rounds * 8 + warp;
+  const int ti = 256 >> sh;   // a tile's rows along x
+  const int j = ((int)blockIdx.x << sh) + ((int)threadIdx.x & ((1 << sh) - 1)), nx = E.n / E.ny_r;
+  const int i1 = min(nx, ((int)blockIdx.y + 1) * rounds * ti);
+  int i = (int)blockIdx.y * rounds * ti + ((int)threadIdx.x >> sh);
   bool ok = j < E.ny_r && i < i1;
   const PatEntry<T>* tb = pat_tab(E, ok ? i * E.ny_r + j : 0);
   uint8_t f = ok ? flags[i * E.ny_r + j] : 0;
@@ -410,10 +431,10 @@ __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
     const int row = i * E.ny_r + j;
     const PatEntry<T>* tc = tb;
     const uint8_t fc = f;
-    ok = i + 8 < i1;
+    ok = i + ti < i1;
     if (ok) {   // the next row's pattern, ahead of its use
-      tb = pat_tab(E, row + 8 * E.ny_r);
-      f = flags[row + 8 * E.ny_r];
+      tb = pat_tab(E, row + ti * E.ny_r);
+      f = flags[row + ti * E.ny_r];
     }
     const double own = (double)r[row];
     double v[1] = {0.0};
@@ -432,7 +453,7 @@ __global__ void __launch_bounds__(256, PCFD_PAT_MINB)
       acc[0] += zn;
       acc[1] += own * zn;
     }
-    i += 8;
+    i += ti;
   }
   block_partial<2>(acc, zpart);
 }

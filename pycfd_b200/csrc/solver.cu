@@ -521,7 +521,7 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
     const int tl = s->tail_level;
     auto product = [&](const Pat<T>& E, const T* s1, const T* s2, T* y, bool from_r) -> int {
       const PatLaunch q = pat_launch(E, s->pat_threads, true);
-      pdl_launch(s, from_r ? k_pat<T, true> : k_pat<T, false>, q.grid, 256, 0, stream, E, q.L, s1, s2,
+      pdl_launch(s, from_r ? k_pat<T, true> : k_pat<T, false>, q.grid, 256, 0, stream, E, q.L, q.sh, s1, s2,
                  (const double*)s->S, s->singular, y);
       CHECK_LAUNCH();
       return 0;
@@ -537,9 +537,9 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
     prof_mark(s, 2, stream);
     {
       const Pat<T>& E = patUp<T>(s)[0];
-      int rounds = 1;
-      const dim3 grid = pat_up0_grid(E, s->pat_threads, s->pat_blocks, &rounds);
-      pdl_launch(s, E.f65 ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds,
+      int rounds = 1, sh = 5;
+      const dim3 grid = pat_up0_grid(E, s->pat_threads, s->pat_blocks, &rounds, &sh);
+      pdl_launch(s, E.f65 ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds, sh,
                  (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, s->singular, (const double*)s->S, z_out, s->zpart);
       s->nz = (int)(grid.x * grid.y);
     }
@@ -2253,8 +2253,8 @@ int pycfd_solver_persistent(pycfd_solver* s, int* ctas) {
 
 int pycfd_solver_form(pycfd_solver* s, int* form) {
   if (!s || !form) return fail(PCFD_E_ARG, "bad arguments");
-  int rounds = 0;
-  if (!s->pup.empty()) pat_up0_grid(s->pup[0], s->pat_threads, s->pat_blocks, &rounds);
+  int rounds = 0, sh = 0;
+  if (!s->pup.empty()) pat_up0_grid(s->pup[0], s->pat_threads, s->pat_blocks, &rounds, &sh);
   form[0] = s->pup.empty() ? 0 : s->tail_level;
   form[1] = rounds;
   form[2] = s->cl_ctas;

@@ -130,4 +130,22 @@ int pt_fits(int nx, int ny, int K) {
   return pat_fits(pat_launch(E, 592 * 256, true));
 }
 
+// Counts in hits[nx * ny] the threads of that launch per row, by the kernel's own index
+// arithmetic (k_pat); returns the parts of a row.
+int pt_cover(int nx, int ny, int K, int* hits) {
+  Pat<double> E{};
+  E.n = nx * ny;
+  E.ny_r = ny;
+  E.K = K;
+  const PatLaunch p = pat_launch(E, 592 * 256, true);
+  for (int by = 0; by < (int)p.grid.y; ++by)
+    for (int bx = 0; bx < (int)p.grid.x; ++bx)
+      for (int t = 0; t < 256; ++t) {
+        int part, i, j;
+        pat_thread(t, bx, by, p.L, p.sh, &part, &i, &j);
+        if (j < ny && i * ny + j < E.n) ++hits[i * ny + j];
+      }
+  return p.L;
+}
+
 }  // extern "C"

@@ -145,8 +145,20 @@ def test_how_many_patterns_are_taken(lib, n, alone, batch):
         lib.pt_free(h)
 
 
-@pytest.mark.parametrize("nx,ny,fits", [(524280, 2, True), (524281, 2, False), (2, 524281, True), (600000, 4, False),
-                                        (8192, 8192, True), (20000, 1, True)])
+@pytest.mark.parametrize("nx", [1, 2, 3, 31, 1000])
+@pytest.mark.parametrize("ny", [1, 2, 3, 4, 5, 15, 16, 17, 31, 32, 33, 64, 100])
+@pytest.mark.parametrize("K", [4, 24, 60, 400])
+def test_tiles_cover_every_row_once(lib, nx, ny, K):
+    """The rows a launch's threads take, each by as many parts as the row has."""
+    out = (C.c_int * (nx * ny))()
+    parts = lib.pt_cover(nx, ny, K, out)
+    assert parts >= 1 and all(v == parts for v in out)
+
+
+@pytest.mark.parametrize("nx,ny,fits", [(524280, 17, True), (524281, 17, False), (2, 524281, True), (600000, 4, True),
+                                        (1048560, 16, True), (1048561, 16, False), (8192, 8192, True),
+                                        (20000, 1, True)])
 def test_grids_of_the_products(lib, nx, ny, fits):
-    """8 rows of tiles along x per block: more than 65,535 blocks along x are not launched."""
+    """A tile is 8 rows along x by 32 along y, 16 by 16 on a grid no wider than that: more
+    than 65,535 tiles along x are not launched."""
     assert bool(lib.pt_fits(nx, ny, 24)) == fits
