@@ -1902,9 +1902,13 @@ int pycfd_momentum_rhs_les(const double* u, const double* v, int nx, int ny, dou
 int pycfd_divergence(const double* u, const double* v, int nx, int ny, double dx, double dy, double* out,
                      void* stream) {
   if (!u || !v || !out || nx < 1 || ny < 1) return fail(PCFD_E_ARG, "bad arguments");
-  // one cell per thread: its four loads are all there is to overlap (a wave of blocks
-  // striding over 16 cells each takes 18 us at 1500x1100 against 15)
-  const dim3 cb(kCellTJ, kCellTI), cg((ny + kCellTJ - 1) / kCellTJ, std::min(65535, (nx + kCellTI - 1) / kCellTI));
+  // 16 blocks per SM, two waves, striding over the rest: enough loads in flight, and few
+  // enough blocks that starting them is no part of the time.  us with 4 per SM / a block for
+  // every 256 cells / this, inputs in L2: 1500x1100 10.4 / 10.4 / 8.4, 60000x64 27 / 31 / 25;
+  // from DRAM: 1500x1100 18.5 / 16.8 / 16.3, 60000x64 37 / 33 / 31, 4096x4096 158 / 137 / 117
+  const dim3 cb(kCellTJ, kCellTI);
+  const int gx = (ny + kCellTJ - 1) / kCellTJ, gy = (nx + kCellTI - 1) / kCellTI;
+  const dim3 cg(gx, std::min(gy, std::max(1, 4 * kWaveBlocks / gx)));
   k_divergence<<<cg, cb, 0, st(stream)>>>(u, v, nx, ny, dx, dy, out);
   CHECK_LAUNCH();
   return 0;

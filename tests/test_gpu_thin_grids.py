@@ -11,6 +11,20 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
+@pytest.mark.parametrize("nx,ny", [(1, 1), (7, 33), (60000, 64), (3, 40000), (2400, 8), (2, 80000)])
+def test_divergence_covers_every_cell(nx, ny):
+    """Fewer and more cells than the launch has threads, along either axis."""
+    from pycfd_b200 import _lib
+    L = _lib.load()
+    u = torch.randn(nx + 3, ny + 2, dtype=torch.float64, device="cuda")
+    v = torch.randn(nx + 2, ny + 3, dtype=torch.float64, device="cuda")
+    out = torch.full((nx, ny), float("nan"), dtype=torch.float64, device="cuda")
+    _lib.check(L.pycfd_divergence(_lib.ptr(u), _lib.ptr(v), nx, ny, 0.25, 0.5, _lib.ptr(out), None))
+    want = (u[2:nx + 2, 1:ny + 1] - u[1:nx + 1, 1:ny + 1]) / 0.25 + (v[1:nx + 1, 2:ny + 2] - v[1:nx + 1, 1:ny + 1]) / 0.5
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)   # powers of two divide exactly; one sum
+
+
 @pytest.mark.parametrize("nx,ny", [(300, 4), (1000, 5), (401, 8), (257, 16), (2000, 17), (5, 700), (4, 2001), (40001, 4)])
 def test_cycle_on_a_thin_grid(nx, ny):
     from pycfd_b200 import _lib
