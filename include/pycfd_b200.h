@@ -311,8 +311,8 @@ int pycfd_step_host(pycfd_solver* s, const double* u0_host, const double* v0_hos
 /* Measurement support (no counterpart in the reference): bracket every eager
  * launch of one kernel with CUDA events on its stream, then read the summed
  * device time.  Ids: 1 CG direction/A-product (k_cg_pq), 2 last fine smoothing
- * sweep of the V-cycle, 3 first fine sweep + residual, 4 coarse-level cluster
- * cycle, 6 momentum predictor, 7 projection correction, 8 whole persistent
+ * sweep of the V-cycle (on row patterns: the level-0 up product), 3 first fine
+ * sweep + residual (no launch on row patterns), 4 coarse-level cluster cycle, 6 momentum predictor, 7 projection correction, 8 whole persistent
  * solve (k_solve_persistent); 0 switches it off.
  * Steps replayed from a recorded graph are not bracketed. */
 int pycfd_profile_kernel(pycfd_solver* s, int kernel_id);
@@ -517,8 +517,10 @@ int pycfd_batch_status(pycfd_batch* b, int* frozen, int* steps, int* iterations,
 /* Measurement support: bracket every eager launch (record = 0) of one kernel
  * kind with CUDA events, then read the summed device time.  Ids: 1 CG
  * direction/A-product, 2 last fine V-cycle sweep (with stencil transfers: and
- * the prolongation onto the fine level), 3 first fine sweep + residual (with
- * stencil transfers: the fused restriction into level 1), 4 coarse levels, 5 CG
+ * the prolongation onto the fine level; on row patterns: the level-0 up
+ * product), 3 first fine sweep + residual (with stencil transfers: the fused
+ * restriction into level 1; no launch on row patterns), 4 coarse levels (on row
+ * patterns: every down product and the up products above level 0), 5 CG
  * update, 6 predictor; 0 off. */
 int pycfd_batch_profile(pycfd_batch* b, int kernel_id);
 int pycfd_batch_profile_read(pycfd_batch* b, double* total_ms, int* launches, void* stream);

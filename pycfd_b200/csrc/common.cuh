@@ -110,12 +110,15 @@ constexpr int kRedThreads = 256;
 
 // Programmatic dependent launch (sm_90+): a kernel launched with the
 // programmatic-serialization attribute may be scheduled while its predecessor
-// is still running.  Every kernel therefore first allows its own successor to be
-// scheduled (which happens once all its blocks have started, so the successor takes
-// only what they leave free), then waits for the predecessor's completion and memory
-// (a no-op without the attribute): launch latency overlaps execution, and what a kernel
-// does between the two -- reading tables that no kernel writes -- overlaps its
-// predecessor.
+// is still running.  Every kernel therefore first waits for the predecessor's
+// completion and memory (a no-op without the attribute), then allows its own
+// successor to be scheduled: launch latency overlaps execution, and what a kernel
+// does before the wait -- reading tables that no kernel writes -- overlaps its
+// predecessor.  The order matters: a kernel past its wait knows that its
+// predecessor is complete, and with it every kernel before that, so buffers can be
+// reused from pass to pass.  Triggered before the wait, a successor could start while
+// the predecessor's predecessor still reads what the successor writes (measured: wrong
+// results).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
@@ -246,8 +249,10 @@ __device__ __forceinline__ void block_total(const double* __restrict__ rows, int
 #pragma unroll
   for (int k = 0; k < NV; ++k) t[k] = all[k];
 }
-// A solver's reduction buffer holds kMaxRedBlocks rows of 8 doubles; the launches with a
-// ticket use the first half, the partials of p.q this part of it.
+// A solver's reduction buffer holds kMaxRedBlocks rows of 8 doubles.  The partials of p.q
+// start at half of it: behind the rows of up to four values that the ticketed launches of a
+// solve leave, since k_cg_xr reads them while its own tickets fill the first half.  (The
+// field statistics use all 8 values of a row; they run between solves.)
 constexpr int kPartPq = 4;
 
 // Fine-level diagonal, accumulated face by face in the reference's order
