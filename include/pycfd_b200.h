@@ -312,8 +312,9 @@ int pycfd_step_host(pycfd_solver* s, const double* u0_host, const double* v0_hos
  * launch of one kernel with CUDA events on its stream, then read the summed
  * device time.  Ids: 1 CG direction/A-product (k_cg_pq), 2 last fine smoothing
  * sweep of the V-cycle (on row patterns: the level-0 up product), 3 first fine
- * sweep + residual (no launch on row patterns), 4 coarse-level cluster cycle, 6 momentum predictor, 7 projection correction, 8 whole persistent
- * solve (k_solve_persistent); 0 switches it off.
+ * sweep + residual (no launch on row patterns), 4 coarse-level cluster cycle,
+ * 6 momentum predictor, 7 projection correction, 8 whole persistent solve
+ * (k_solve_persistent); 0 switches it off.
  * Steps replayed from a recorded graph are not bracketed. */
 int pycfd_profile_kernel(pycfd_solver* s, int kernel_id);
 /* CTAs of the cooperative launch that runs each CG / MG-PCG solve whole

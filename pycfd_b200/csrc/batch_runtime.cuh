@@ -105,17 +105,16 @@ int upload_hier(pycfd_batch* B, const pycfd_solver_desc* d, const PatCycle<T>* c
     const pycfd_mg_level& up = d->levels[l - 1];
     Level& L = (*keep)[l];
     L.n = in.n;
-    if (cyc) continue;
     const bool coarsest = l == Lv - 1;
+    TRY(check_level(in, l, coarsest));
+    if (cyc) continue;
     DevEll<T> A, P, R;
     T* wd = nullptr;
     if (!coarsest) {
-      if (!in.a_indptr || !in.weighted_dinv) return fail(PCFD_E_ARG, "level %d lacks A", l);
       TRY(make_ell(B->mem, &A, in.n, in.a_indptr, in.a_indices, in.a_data));
       std::vector<T> w(in.weighted_dinv, in.weighted_dinv + in.n);
       TRY(upload(B->mem, &wd, w.data(), w.size()));
     }
-    if (!in.p_indptr) return fail(PCFD_E_ARG, "level %d lacks P", l);
     TRY(make_ell(B->mem, &P, up.n, in.p_indptr, in.p_indices, in.p_data));
     std::vector<int64_t> tp;
     std::vector<int32_t> ti;

@@ -250,6 +250,13 @@ int upload(pycfd_solver* s, T** p, const T* host, size_t count) {
   return 0;
 }
 
+// What a level l >= 1 of a descriptor must carry, whichever form of the cycle reads it.
+int check_level(const pycfd_mg_level& in, int l, bool coarsest) {
+  if (!coarsest && (!in.a_indptr || !in.weighted_dinv)) return fail(PCFD_E_ARG, "level %d lacks A", l);
+  if (!in.p_indptr) return fail(PCFD_E_ARG, "level %d lacks P", l);
+  return 0;
+}
+
 // CSR -> ELL (entries of a row sorted by column) in the layout its lane count wants.
 template <class T>
 int make_ell(pycfd_solver* s, DevEll<T>* E, int n, const int64_t* indptr, const int32_t* idx,
@@ -1705,10 +1712,10 @@ static int solver_create(const pycfd_solver_desc* d, bool member, pycfd_solver**
           (rc = dalloc(s, &L.d.res, L.n)) || (rc = dalloc(s, &L.f.b, L.n)) || (rc = dalloc(s, &L.f.xa, L.n)) ||
           (rc = dalloc(s, &L.f.xb, L.n)) || (rc = dalloc(s, &L.f.res, L.n)))
         return bail(rc);
+      if (l >= 1 && (rc = check_level(in, l, coarsest))) return bail(rc);
       if (l >= 1 && !pats) {
         const pycfd_mg_level& up = d->levels[l - 1];
         if (!coarsest) {
-          if (!in.a_indptr || !in.weighted_dinv) return bail(fail(PCFD_E_ARG, "level %d lacks A", l));
           if ((rc = make_ell(s, &L.A, L.n, in.a_indptr, in.a_indices, in.a_data)) ||
               (rc = make_ell(s, &L.Af, L.n, in.a_indptr, in.a_indices, in.a_data)))
             return bail(rc);
@@ -1716,7 +1723,6 @@ static int solver_create(const pycfd_solver_desc* d, bool member, pycfd_solver**
           if ((rc = upload(s, &L.wd, in.weighted_dinv, L.n)) || (rc = upload(s, &L.wdf, wf.data(), L.n)))
             return bail(rc);
         }
-        if (!in.p_indptr) return bail(fail(PCFD_E_ARG, "level %d lacks P", l));
         if ((rc = make_ell(s, &L.P, up.n, in.p_indptr, in.p_indices, in.p_data)) ||
             (rc = make_ell(s, &L.Pf, up.n, in.p_indptr, in.p_indices, in.p_data)))
           return bail(rc);

@@ -137,3 +137,24 @@ def test_launch_counts_of_recorded_solves_beside_other_threads():
 
     one_by_one = total(False)
     assert one_by_one > 0 and total(True) == one_by_one
+
+
+@pytest.mark.parametrize("field", ["a_indptr", "weighted_dinv", "p_indptr"])
+def test_incomplete_levels_are_refused_whatever_the_form(field):
+    """A level below the dense tail without its operator: read by no kernel of the pattern
+    form, and refused by it as by the stored one."""
+    import ctypes as C
+    from pycfd_b200 import _lib
+    from pycfd_b200.config import PressureSolver
+    from pycfd_b200.solver import GpuOptions, native_desc
+    L = _lib.load()
+    s = _solver(_cfg(128, 128))
+    assert s.form()["pattern_levels"] == 2 and len(s._levels) > 4
+    for fused in (True, False):
+        d, keep = native_desc(s.config, s.mesh, s.boundaries, s.solid, False, (), PressureSolver.MGCG,
+                              GpuOptions(fused_restriction=fused), s._levels, s._cinv)
+        e = d.levels[3]
+        setattr(e, field, C.cast(C.c_void_p(0), type(getattr(e, field))))
+        h = C.c_void_p()
+        with pytest.raises(ValueError, match="level 3 lacks"):
+            _lib.check(L.pycfd_solver_create(C.byref(d), C.byref(h)))
