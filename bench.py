@@ -465,7 +465,8 @@ def run_batch(args, world, rank, local):
                             {"ms": v[0], "launches": v[1],
                              "gb_s": (v[2] / (v[0] / 1e3) / 1e9) if v[0] > 0 and v[2] else None}
                             for k, v in prof.items()},
-                "traffic_source": "profiles/roofline_traffic.json (one ncu capture of this kernel)"}
+                "traffic_source": "profiles/roofline_traffic.json (one ncu capture of this kernel)"
+                                  if traffic is not None else None}
         if args.parts > 1:
             # the same kernel kinds at full size: the whole batch in one engine, so every
             # launch covers every cavity (the timed step's parts launch a quarter each)

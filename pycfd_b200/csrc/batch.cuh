@@ -2048,8 +2048,9 @@ __global__ void __launch_bounds__(kBThreads, PCFD_BELL_MINB) k_b_ellg(const BPro
 // problems: a row's entries are read from the pattern table once for the group, its
 // gathers run along y over adjacent rows, and L > 1 splits the entries of the wide,
 // short levels over L parts of the block (each warp still covers 32 adjacent rows).
-// What bounds these launches is latency (dependent loads at the start of a block, gathers
-// at 40 % of the warp slots) and, at level 0, the instructions per gather; the grouped ELL
+// What bounds these launches is L1 (60 to 70 % of its throughput on the coarse levels of 256
+// cavities) and latency: dependent loads at the start of a block, and at level 0, where 34 %
+// of the warp slots are in use (80 registers), the block's start and close.  The grouped ELL
 // phases they replace read 8 bytes per entry and row from L2 with the row's entries spread
 // over a warp.  Per launch on 256 cavities in one engine (us): down onto level 1 60 -> 35,
 // onto 2 30 -> 22; level 1 up 76 (two launches) -> 37, level 2 up 58 -> 27; level 0 with
