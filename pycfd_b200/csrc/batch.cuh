@@ -2277,7 +2277,7 @@ __global__ void __launch_bounds__(kBThreads, 3)
   __shared__ BPatGroup<T, GM> G;
   __shared__ unsigned closing;
   const Pat<T> E = H.up[0];
-  const bool usual = E.f65 != 0;
+  const bool usual = pat_is_65(E);
   const int KT = E.K + E.K2;
   const int rb = e.y >> 12;
   const uint8_t* __restrict__ flags = probs[sprobs[H.sp0]].flags;   // the structure's

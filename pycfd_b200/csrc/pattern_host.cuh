@@ -243,8 +243,7 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
     K = std::max<int>(K, (int)(A.ptr[r + 1] - A.ptr[r]));
     if (B) K2 = std::max<int>(K2, (int)(B->ptr[r + 1] - B->ptr[r]));
   }
-  E.f65 = up0 && K == 6 && K2 == 5;
-  if (!E.f65) {   // units of four entries (pattern.cuh)
+  if (!(up0 && K == 6 && K2 == 5)) {   // units of four entries (pattern.cuh)
     K = (K + kPatUnit - 1) / kPatUnit * kPatUnit;
     K2 = (K2 + kPatUnit - 1) / kPatUnit * kPatUnit;
   }

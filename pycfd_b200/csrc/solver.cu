@@ -546,7 +546,7 @@ int vcycle_pcg(pycfd_solver* s, const T* r, T* z_out, cudaStream_t stream) {
       const Pat<T>& E = patUp<T>(s)[0];
       int rounds = 1, sh = 5;
       const dim3 grid = pat_up0_grid(E, s->pat_threads, s->pat_blocks, &rounds, &sh);
-      pdl_launch(s, E.f65 ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds, sh,
+      pdl_launch(s, pat_is_65(E) ? k_pat_up0<T, true> : k_pat_up0<T, false>, grid, 256, 0, stream, E, rounds, sh,
                  (const T*)lvB<T>(s->lv[1]).xa, r, (const uint8_t*)s->flags, s->singular, (const double*)s->S, z_out, s->zpart);
       s->nz = (int)(grid.x * grid.y);
     }

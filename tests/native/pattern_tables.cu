@@ -69,7 +69,7 @@ void apply(const Pat<T>& E0, const PatHost<T>& h, bool level0_up, int parts, con
     double sum = 0.0;
     if (level0_up) {
       double acc[1] = {0.0};
-      if (E.f65) pat_whole<true, 1>(E, tb, row, xa, xb, acc);
+      if (pat_is_65(E)) pat_whole<true, 1>(E, tb, row, xa, xb, acc);
       else pat_whole<false, 1>(E, tb, row, xa, xb, acc);
       sum = acc[0];
     } else {
@@ -109,7 +109,7 @@ void pt_info(void* h, int single, int l, int up, int* out) {
     out[1] = p.v.K2;
     out[2] = p.v.n;
     out[3] = (int)(p.tab.size() / (p.v.K + p.v.K2));
-    out[4] = p.v.f65;
+    out[4] = pat_is_65(p.v);
   };
   if (single) fill(pick(((Cycle*)h)->f, l, up));
   else fill(pick(((Cycle*)h)->d, l, up));
