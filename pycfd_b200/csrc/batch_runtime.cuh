@@ -206,7 +206,7 @@ int batch_build(pycfd_batch* B, const pycfd_solver_desc* descs, const int* struc
       std::vector<std::function<bool()>> own;
       pat[h] = asked && d.n_levels >= 2 && d.n_levels <= kBMaxLevels && d.levels && d.coarsest_inverse &&
                d.levels[0].n == d.nx * d.ny &&
-               pat_tasks<T>(d.levels, b_closed_at(&d), true, B->solvers[leaders[h]]->hflags.data(), &cyc[h], &own);
+               pat_tasks<T>(d.levels, b_closed_at(&d), kPatBatch, B->solvers[leaders[h]]->hflags.data(), &cyc[h], &own);
       for (auto& t : own)
         if (pat[h]) tasks.push_back([&pat, h, t]() {
           bool ok = false;

@@ -214,16 +214,13 @@ struct PatHost {
   std::vector<PatEntry<T>> tab;
 };
 
-// The rows of A (and of B, the second source) as patterns, or false where there are
-// more than the rule allows.  liveA, liveB: entries at columns whose source value is
-// zero by definition are dropped.
 // How many patterns pay, measured on masks with nearly as many patterns as rows (one solid
 // cell at a random place of every 4 x 4 block), ms per step.
 // One problem alone: at most one per 4 rows on levels over 16384 rows, where a row with a
 // pattern of its own reads its table uncoalesced (FP64 400x400: 2.3 with the stored
 // operators, 2.6 on patterns; 500x500 2.8 and 2.9); smaller levels stay in L1 and L2 whatever
 // their patterns (256x256 1.63 stored, 1.56 on patterns, 64x64 1.06 and 0.87).
-// any (a batch): no limit but the 65,535 a row can name.  Against the default level-by-level
+// dense (a batch): no limit but the 65,535 a row can name.  Against the default level-by-level
 // cycle the patterns are always faster (FP64 / mixed, each problem its own mask: 8 of 256x256
 // 8.4 / 8.7 -> 7.3 / 6.6, 24 of 256x256 17.3 / 15.9 -> 15.7 / 14.1, 8 of 400x400 13.6 / 13.6
 // -> 12.8 / 12.4, 64 of 128x128 11.6 / 10.2 -> 11.2 / 9.3).  Against the fused down sweep on
@@ -232,9 +229,32 @@ struct PatHost {
 // 128x128 10.6 / 9.0 -> 11.2 / 9.3, 8 of 400x400 12.4 / 11.8 -> 12.8 / 12.4); a limit per
 // structure would not see that, and one per engine would tie a problem's route to its
 // neighbours.
+//
+// How wide rows may be: a level above the closing one whose widest row of A has more than
+// `widest` entries keeps its structure on stored operators.  Uniform cells of aspect 1.5 and
+// more coarsen along one axis at a time, and their rows grow to hundreds and thousands of
+// entries (square cells stay near 100): the products grow with the square of the width, hardly
+// two rows are equal, and a row's table is read by one lane at a stride of the whole row.
+// ms, stored -> patterns.  Solves of one problem, FP64 / mixed: width 225 (256x256) 0.53 / 0.61
+// -> 0.51 / 0.52; 349 (192x192) 0.69 / 0.66 -> 0.68 / 0.59, (256x256) 0.98 / 1.01 -> 0.91 /
+// 0.72, (256x128) 0.78 / 0.76 -> 0.84 / 0.72; 425 (160x160) 0.85 / 0.77 -> 1.01 / 0.80; 1155
+// (400x100) 0.92 / 1.09 -> 1.48 / 1.29; 1577 (512x256) 2.48 -> 3.12.  Steps of 64 problems,
+// default down sweep (and the fused one on stored operators): width 225 (160x160) 7.5 / 7.9
+// (6.3 / 6.8) -> 6.4 / 6.1; 349 (96x96) 5.7 / 5.0 (4.7 / 4.2) -> 5.9 / 4.7, and 256 of them
+// 13.4 / 10.9 (11.7 / 9.2) -> 16.9 / 11.9; 1361 (160x160) 16.8 / 13.8 (14.1 / 11.6) -> 22.8 /
+// 18.8.
+struct PatRule {
+  bool dense;
+  int widest;
+};
+constexpr PatRule kPatAlone{false, 400}, kPatBatch{true, 256};
+
+// The rows of A (and of B, the second source) as patterns, or false where there are
+// more than the rule allows.  liveA, liveB: entries at columns whose source value is
+// zero by definition are dropped.
 // up0: the level-0 up product, whose kernels read 6 + 5 entries without padding.
 template <class T>
-bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t* liveB, bool up0, bool any,
+bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t* liveB, bool up0, bool dense,
                PatHost<T>* out) {
   Pat<T>& E = out->v;
   const int n = A.n;
@@ -248,7 +268,7 @@ bool pat_build(const CsrV& A, const uint8_t* liveA, const CsrV* B, const uint8_t
     K2 = (K2 + kPatUnit - 1) / kPatUnit * kPatUnit;
   }
   const int KT = K + K2;
-  const size_t most = std::min<size_t>(65535, n > 16384 && !any ? (size_t)n / 4 : (size_t)n);
+  const size_t most = std::min<size_t>(65535, n > 16384 && !dense ? (size_t)n / 4 : (size_t)n);
   E.K = K;
   E.K2 = K2;
   out->pid.resize(n);
@@ -317,7 +337,7 @@ struct PatCycle {
 // Appends the cycle's work to `tasks` (largest level first); false where its shapes
 // rule patterns out.  out and lv stay as they are until the tasks have run.
 template <class T>
-bool pat_tasks(const pycfd_mg_level* lv, int t, bool any, const uint8_t* flags, PatCycle<T>* out,
+bool pat_tasks(const pycfd_mg_level* lv, int t, PatRule rule, const uint8_t* flags, PatCycle<T>* out,
                std::vector<std::function<bool()>>* tasks) {
   out->dn.resize(t + 1);
   out->up.resize(t + 1);
@@ -326,6 +346,8 @@ bool pat_tasks(const pycfd_mg_level* lv, int t, bool any, const uint8_t* flags, 
   for (int l = 0; l < t; ++l) {
     const pycfd_mg_level *f = lv + l, *c = lv + l + 1;
     if (!f->a_indptr || !f->weighted_dinv || !c->p_indptr) return false;
+    for (int r = 0; r < f->n; ++r)
+      if (f->a_indptr[r + 1] - f->a_indptr[r] > rule.widest) return false;
     PatHost<T>*m = &out->dn[l + 1], *q = &out->up[l];
     if (!pat_shape(&m->v, c->n, c->shape_x, c->shape_y, f->n, f->shape_x, f->shape_y) ||
         !pat_shape(&q->v, f->n, f->shape_x, f->shape_y, c->n, c->shape_x, c->shape_y))
@@ -335,9 +357,9 @@ bool pat_tasks(const pycfd_mg_level* lv, int t, bool any, const uint8_t* flags, 
       Csr Q, G;
       up_products(*f, *c, &Q, &G);
       const CsrV g = G;
-      return pat_build<T>(Q, nullptr, &g, live, l == 0, any, q);
+      return pat_build<T>(Q, nullptr, &g, live, l == 0, rule.dense, q);
     });
-    tasks->push_back([=]() { return pat_build<T>(down_product(*f, *c), live, nullptr, nullptr, false, any, m); });
+    tasks->push_back([=]() { return pat_build<T>(down_product(*f, *c), live, nullptr, nullptr, false, rule.dense, m); });
   }
   return true;
 }

@@ -1027,8 +1027,8 @@ bool pattern_cycle(pycfd_solver* s, const pycfd_solver_desc* d, int* rc) {
   PatCycle<double> cd;
   PatCycle<float> cf;
   std::vector<std::function<bool()>> tasks;
-  if (!pat_tasks<double>(d->levels, t, false, s->hflags.data(), &cd, &tasks)) return false;
-  if (mixed && !pat_tasks<float>(d->levels, t, false, s->hflags.data(), &cf, &tasks)) return false;
+  if (!pat_tasks<double>(d->levels, t, kPatAlone, s->hflags.data(), &cd, &tasks)) return false;
+  if (mixed && !pat_tasks<float>(d->levels, t, kPatAlone, s->hflags.data(), &cf, &tasks)) return false;
   if (!run_tasks(tasks)) return false;
   for (int l = 1; l <= t; ++l)
     if (!pat_fits(pat_launch(cd.dn[l].v, s->pat_threads, true)) ||

@@ -48,9 +48,9 @@ struct Cycle {
 };
 
 template <class T>
-bool build(const pycfd_mg_level* lv, int t, bool any, const uint8_t* flags, PatCycle<T>* c) {
+bool build(const pycfd_mg_level* lv, int t, PatRule rule, const uint8_t* flags, PatCycle<T>* c) {
   std::vector<std::function<bool()>> tasks;
-  return pat_tasks<T>(lv, t, any, flags, c, &tasks) && run_tasks(tasks);
+  return pat_tasks<T>(lv, t, rule, flags, c, &tasks) && run_tasks(tasks);
 }
 
 // y = E s1 (+ E2 s2) as the kernels walk a row: level 0's up product whole, any other by
@@ -90,13 +90,14 @@ const PatHost<T>& pick(const PatCycle<T>& c, int l, int up) { return up ? c.up[l
 
 extern "C" {
 
-// The products of levels 0 .. t; solvable: one byte per fine cell.
-void* pt_build(const pycfd_mg_level* lv, int t, int any, const uint8_t* solvable) {
+// The products of levels 0 .. t by the rule of a batch or of a problem alone; solvable: one
+// byte per fine cell.
+void* pt_build(const pycfd_mg_level* lv, int t, int batch, const uint8_t* solvable) {
   std::unique_ptr<Cycle> c(new Cycle());
   std::vector<uint8_t> flags(lv[0].n);
   for (int k = 0; k < lv[0].n; ++k) flags[k] = solvable[k] ? F_SOLV : 0;
-  c->ok_d = build<double>(lv, t, any != 0, flags.data(), &c->d);
-  c->ok_f = build<float>(lv, t, any != 0, flags.data(), &c->f);
+  c->ok_d = build<double>(lv, t, batch ? kPatBatch : kPatAlone, flags.data(), &c->d);
+  c->ok_f = build<float>(lv, t, batch ? kPatBatch : kPatAlone, flags.data(), &c->f);
   return c.release();
 }
 void pt_free(void* h) { delete (Cycle*)h; }

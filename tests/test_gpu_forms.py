@@ -158,3 +158,20 @@ def test_incomplete_levels_are_refused_whatever_the_form(field):
         h = C.c_void_p()
         with pytest.raises(ValueError, match="level 3 lacks"):
             _lib.check(L.pycfd_solver_create(C.byref(d), C.byref(h)))
+
+
+def test_wide_rows_keep_stored_operators():
+    """Cells of aspect 2.2 and 1.5: rows of 349 and 576 entries above the closing level."""
+    from pycfd_b200.batch import BatchedSolver, BatchOptions
+    assert _solver(_cfg(192, 192, lx=2.2)).form()["pattern_levels"] > 0
+    assert _solver(_cfg(192, 192, lx=1.5)).form()["pattern_levels"] == 0
+    cfgs = [_cfg(96, 96, lx=lx, adaptive_dt=False, dt=1e-3, t_end=10.0) for lx in (1.0, 3.0, 2.2, 1.5)]
+    b = BatchedSolver(cfgs, BatchOptions())
+    assert (b.form()["pattern_structures"], b.form()["stored_structures"]) == (2, 2)
+    g = BatchedSolver(cfgs, BatchOptions(ell_group=1))
+    for x in (b, g):
+        x.step(3)
+        assert not x.status()["status"].any()
+    for f, h in zip(b.fields, g.fields):
+        for p, q in zip(f.numpy(), h.numpy()):
+            assert np.abs(p - q).max() <= 1e-8 * max(np.abs(a).max() for a in h.numpy())

@@ -45,9 +45,10 @@ def circle(nx, ny):
     return (x - 0.4 * nx) ** 2 + (y - 0.5 * ny) ** 2 < (0.2 * min(nx, ny)) ** 2
 
 
-def problem(nx, ny, solid, ratio, bc=None):
+def problem(nx, ny, solid, ratio, bc=None, aspect=1.0):
     """(levels, closing level, descriptor, what it points to, solvable cells)."""
-    cfg = cases.to_config(dict(nx=nx, ny=ny, lx=nx / 64.0, ly=ny / 64.0, re=100.0, pressure_solver="mgcg",
+    cfg = cases.to_config(dict(nx=nx, ny=ny, lx=aspect * nx / 64.0, ly=ny / 64.0, re=100.0,
+                               pressure_solver="mgcg",
                                boundary_config=bc or cases.bcs()), SimulationConfig, BCSpec, BCKind)
     mesh = StructuredMesh.from_config(cfg)
     bnd = BoundaryInfo(cfg.boundary_config, mesh)
@@ -162,3 +163,19 @@ def test_grids_of_the_products(lib, nx, ny, fits):
     """A tile is 8 rows along x by 32 along y, 16 by 16 on a grid no wider than that: more
     than 65,535 tiles along x are not launched."""
     assert bool(lib.pt_fits(nx, ny, 24)) == fits
+
+
+@pytest.mark.parametrize("nx,ny,aspect,ratio,width,alone,batch", [
+    (96, 96, 1.0, 16.0, 37, True, True), (96, 96, 3.0, 16.0, 225, True, True), (96, 96, 2.2, 16.0, 349, True, False),
+    (96, 96, 6.0, 16.0, 425, False, False), (96, 96, 1.5, 16.0, 576, False, False),
+    (128, 128, 2.0, None, 79, True, True)])
+def test_wide_rows_keep_stored_operators(lib, nx, ny, aspect, ratio, width, alone, batch):
+    """Anisotropic cells: the widest row of A on a level above the closing one decides,
+    at 400 entries for a problem alone and at 256 in a batch."""
+    levels, t, d, keep, solvable = problem(nx, ny, None, ratio, aspect=aspect)
+    widest = max(int(np.diff(lv.A.tocsr().indptr).max()) for lv in levels[:t])
+    assert widest == width
+    for b, want in ((0, alone), (1, batch)):
+        h = lib.pt_build(C.cast(d.levels, C.c_void_p), t, b, solvable.ctypes.data)
+        assert bool(lib.pt_ok(h, 0)) == bool(lib.pt_ok(h, 1)) == want
+        lib.pt_free(h)
